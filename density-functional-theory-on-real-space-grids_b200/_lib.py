@@ -112,6 +112,12 @@ SIGNATURES: dict[str, tuple] = {
     "cdftb_quadrature_interpolate_grouped_f64": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p,
                                                          c_void_p, c_int64, c_void_p, c_int, c_int64, c_void_p,
                                                          c_int64, c_void_p, c_int64, c_void_p]),
+    "cdftb_cell_plan_bytes": (c_int64, [c_int64, c_int, c_int, c_int, c_void_p]),
+    "cdftb_cell_plan_build": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p,
+                                      c_void_p, c_int64, c_void_p]),
+    "cdftb_lift_cells_scratch_bytes": (c_int64, [c_int64, c_int, c_int, c_int, c_void_p, c_int]),
+    "cdftb_quadrature_lift_cells_f64": (c_int, [c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_void_p,
+                                                c_int, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p]),
     "cdftb_lift_segments_capacity": (c_int64, [c_int64, c_int64]),
     "cdftb_lift_segments_scratch_bytes": (c_int64, [c_int64]),
     "cdftb_lift_plan_segments": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int64, c_void_p, c_int64,

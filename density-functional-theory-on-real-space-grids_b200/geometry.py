@@ -270,7 +270,7 @@ class CuspQuadrature:
         call("cdftb_geometry_node_fields", n_atoms, _hptr(factor._charges_h), _hptr(factor._positions_h),
              _hptr(self.sphere_rows), cell_width, ptr(self.points), ptr(owner_d), ptr(base_d), m, ptr(self.partition),
              ptr(self.weights), ptr(self.f2), ptr(self.grad_u), ptr(self.transformed_potential), stream)
-        # interpolant stencils and the CSR of its transpose
+        # interpolant stencils
         self.base = torch.empty((m, 3), dtype=torch.int32, device=dev)
         self.w1d = torch.empty((m, 24), **f)
         bad = _flag(dev)
@@ -279,32 +279,23 @@ class CuspQuadrature:
         if int(bad.item()):
             raise ValueError("an interpolation stencil reaches outside the grid; the sphere radius bound is wrong")
         n = grid.n_points
-        self.row_ptr = torch.empty(n + 1, dtype=torch.int64, device=dev)
-        self.col = torch.empty(m * 512, dtype=torch.int32, device=dev)
-        nbytes = _lib.library().cdftb_lift_plan_scratch_bytes(m, n)
-        scratch = torch.empty(max(nbytes, 8), dtype=torch.uint8, device=dev)
-        call("cdftb_lift_plan_build", ptr(self.base), m, *grid.shape, ptr(self.row_ptr), ptr(self.col), ptr(scratch),
-             scratch.numel(), stream)
-        del scratch
-        # the weight of every entry of L^T, formed once (the lifts then stream (col, value) pairs)
-        self.lift_values = torch.empty(m * 512, dtype=torch.float64, device=dev)
-        call("cdftb_lift_plan_values_f64", ptr(self.base), ptr(self.w1d), ptr(self.row_ptr), ptr(self.col),
-             *grid.shape, ptr(self.lift_values), stream)
-        # the rows of L^T cut into segments of at most 256 entries (the many-field lift's work units)
-        lib = _lib.library()
-        self.seg_capacity = lib.cdftb_lift_segments_capacity(m, n)
-        self.seg_ptr = torch.empty(n + 1, dtype=torch.int32, device=dev)
-        self.seg_row = torch.empty(self.seg_capacity, dtype=torch.int32, device=dev)
-        seg_scratch = torch.empty(lib.cdftb_lift_segments_scratch_bytes(n), dtype=torch.uint8, device=dev)
-        call("cdftb_lift_plan_segments", ptr(self.row_ptr), *grid.shape, ptr(self.seg_ptr), ptr(self.seg_row),
-             self.seg_capacity, ptr(seg_scratch), seg_scratch.numel(), stream)
-        del seg_scratch
         # the nodes grouped by base cell (nodes of a group read the same 8^3 box): the many-field
         # interpolant reads each box once per group instead of once per node
         key = (self.base[:, 0].to(torch.int64) * grid.shape[1] + self.base[:, 1]) * grid.shape[2] + self.base[:, 2]
         key, order = torch.sort(key, stable=True)
         _, counts = torch.unique_consecutive(key, return_counts=True)
         self.group_nodes = order.to(torch.int32).contiguous()
+        # the cells that may hold nodes: the spheres' box
+        centres, radii = self.sphere_rows[:, :3], self.sphere_rows[:, 3:4]
+        low = np.floor(((centres - radii).min(axis=0) - origin) / h)
+        high = np.floor(((centres + radii).max(axis=0) - origin) / h)
+        top = np.asarray(grid.shape) - 1
+        self._cell_box = np.concatenate([np.clip(low, 0, top), np.clip(high, 0, top)]).astype(np.int32)
+        box = _hptr(self._cell_box)
+        nbytes = _lib.library().cdftb_cell_plan_bytes(m, *grid.shape, box)
+        self._cell_plan = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
+        call("cdftb_cell_plan_build", ptr(self.base), ptr(self.w1d), ptr(self.group_nodes), ptr(key), m, *grid.shape,
+             box, ptr(self._cell_plan), nbytes, stream)
         # work items of at most GROUP_BATCH nodes of one cell (a cell near a nucleus holds up to ~80
         # nodes): one warp each, so that a crowded cell does not hold up the launch
         starts = torch.cumsum(counts, 0) - counts
@@ -360,6 +351,35 @@ class CuspQuadrature:
         return out
 
     # --- interpolation and its transpose (quadrature.py:613-650) ---
+    #: The entry lists of L^T (cdftb_lift_plan_build and its values and segments), which the C entry points
+    #: over them take and the lift here does not: built when first read.
+    _CSR = ("row_ptr", "col", "lift_values", "seg_ptr", "seg_row", "seg_capacity")
+
+    def __getattr__(self, name):
+        if name not in CuspQuadrature._CSR or "w1d" not in self.__dict__:
+            raise AttributeError(name)
+        lib = _lib.library()
+        n, m, dev = self.grid.n_points, self.n_nodes, self.w1d.device
+        shape, stream = self.grid.shape, stream_handle(dev)
+        row_ptr = torch.empty(n + 1, dtype=torch.int64, device=dev)
+        col = torch.empty(m * 512, dtype=torch.int32, device=dev)
+        scratch = torch.empty(max(lib.cdftb_lift_plan_scratch_bytes(m, n), 8), dtype=torch.uint8, device=dev)
+        call("cdftb_lift_plan_build", ptr(self.base), m, *shape, ptr(row_ptr), ptr(col), ptr(scratch), scratch.numel(),
+             stream)
+        values = torch.empty(m * 512, dtype=torch.float64, device=dev)
+        call("cdftb_lift_plan_values_f64", ptr(self.base), ptr(self.w1d), ptr(row_ptr), ptr(col), *shape, ptr(values),
+             stream)
+        # the rows cut into segments of at most 256 entries
+        capacity = lib.cdftb_lift_segments_capacity(m, n)
+        seg_ptr = torch.empty(n + 1, dtype=torch.int32, device=dev)
+        seg_row = torch.empty(capacity, dtype=torch.int32, device=dev)
+        scratch = torch.empty(lib.cdftb_lift_segments_scratch_bytes(n), dtype=torch.uint8, device=dev)
+        call("cdftb_lift_plan_segments", ptr(row_ptr), *shape, ptr(seg_ptr), ptr(seg_row), capacity, ptr(scratch),
+             scratch.numel(), stream)
+        self.row_ptr, self.col, self.lift_values = row_ptr, col, values
+        self.seg_ptr, self.seg_row, self.seg_capacity = seg_ptr, seg_row, capacity
+        return self.__dict__[name]
+
     #: From this many fields on, L and L^T run one pass per 32 fields (the batched systems).
     MANY_FIELDS = 8
     #: Nodes of one cell per warp of the grouped interpolant (GROUP_BATCH in csrc/quadrature.cu).
@@ -385,14 +405,12 @@ class CuspQuadrature:
     def _lift_raw(self, x: torch.Tensor, nf: int) -> torch.Tensor:
         n = self.grid.n_points
         out = torch.empty((nf, n), dtype=torch.float64, device=x.device)
-        if nf >= self.MANY_FIELDS:
-            scratch = self._many_scratch(x.device)
-            call("cdftb_quadrature_lift_many_f64", ptr(self.row_ptr), ptr(self.col), ptr(self.lift_values),
-                 ptr(self.seg_ptr), ptr(self.seg_row), self.seg_capacity, *self.grid.shape, self.n_nodes, ptr(x), nf,
-                 self.n_nodes, ptr(out), n, ptr(scratch), scratch.numel(), stream_handle(x.device))
-            return out
-        call("cdftb_quadrature_lift_f64", ptr(self.base), ptr(self.w1d), ptr(self.row_ptr), ptr(self.col),
-             ptr(self.lift_values), *self.grid.shape, ptr(x), nf, self.n_nodes, ptr(out), n, stream_handle(x.device))
+        box = _hptr(self._cell_box)
+        nbytes = _lib.library().cdftb_lift_cells_scratch_bytes(self.n_nodes, *self.grid.shape, box, nf)
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+        call("cdftb_quadrature_lift_cells_f64", ptr(self._cell_plan), self._cell_plan.numel(), self.n_nodes,
+             *self.grid.shape, box, ptr(x), nf, self.n_nodes, ptr(out), n, ptr(scratch), nbytes,
+             stream_handle(x.device))
         return out
 
     def interpolate(self, field: torch.Tensor) -> torch.Tensor:

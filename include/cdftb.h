@@ -364,6 +364,23 @@ int cdftb_quadrature_lift_many_f64(const long long* row_ptr, const int* col, con
                                    const double* node_values, int nf, int64_t x_stride, double* out,
                                    int64_t out_stride, void* scratch, int64_t scratch_bytes, cdftb_stream_t stream);
 
+/* L^T without its list of entries, over nodes sorted by base cell (keys: (x ny + y) nz + z of the
+ * cell, int64, ascending; order: the node of every sorted position). cell_box: 6 host ints, per axis
+ * the lowest and then the highest cell index that may hold a node. The plan (cdftb_cell_plan_bytes of
+ * device memory, 16-byte aligned) keeps each cell's first node, the sorted nodes' weights and the work
+ * items of the two kernels. Results equal cdftb_quadrature_lift_f64's up to the order of the sums
+ * (~1e-16 relative). From CDFTB_LIFT_CELLS_MANY fields on, a pass takes 32 fields. */
+#define CDFTB_LIFT_CELLS_MANY 8
+int64_t cdftb_cell_plan_bytes(int64_t m, int nx, int ny, int nz, const int* cell_box);
+int cdftb_cell_plan_build(const int* base, const double* w1d, const int* order, const int64_t* keys, int64_t m,
+                          int nx, int ny, int nz, const int* cell_box, void* plan, int64_t plan_bytes,
+                          cdftb_stream_t stream);
+int64_t cdftb_lift_cells_scratch_bytes(int64_t m, int nx, int ny, int nz, const int* cell_box, int nf);
+int cdftb_quadrature_lift_cells_f64(const void* plan, int64_t plan_bytes, int64_t m, int nx, int ny, int nz,
+                                    const int* cell_box, const double* node_values, int nf, int64_t x_stride,
+                                    double* out, int64_t out_stride, void* scratch, int64_t scratch_bytes,
+                                    cdftb_stream_t stream);
+
 /* ---- (c2, s1) the Kohn-Sham potentials (src/cdft/scf/step.py:224-313) ---- */
 
 /* c = S^{-1} (nucleus_f2 * rho(R_a)) per system (step.py:240-242). */
