@@ -112,6 +112,9 @@ SIGNATURES: dict[str, tuple] = {
     "cdftb_quadrature_interpolate_grouped_f64": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p,
                                                          c_void_p, c_int64, c_void_p, c_int, c_int64, c_void_p,
                                                          c_int64, c_void_p, c_int64, c_void_p]),
+    "cdftb_quadrature_interpolate_groups_f64": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p,
+                                                        c_void_p, c_int64, c_void_p, c_int, c_int64, c_void_p,
+                                                        c_int64, c_void_p]),
     "cdftb_cell_plan_bytes": (c_int64, [c_int64, c_int, c_int, c_int, c_void_p]),
     "cdftb_cell_plan_build": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p,
                                       c_void_p, c_int64, c_void_p]),

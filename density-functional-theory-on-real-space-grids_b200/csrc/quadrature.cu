@@ -3,7 +3,7 @@
 // its three 8-point one-dimensional weight vectors, and a tap's value is (wx * wy) * wz, the
 // product the reference stores in its CSR (src/cdft/operators/quadrature.py:56-93, 506-650).
 //
-// interpolate: one warp per node gathers its 512 taps (8 contiguous z values per row).
+// interpolate: one warp per node, or per group of up to four nodes of one cell, gathers the 512 taps.
 // lift: the transpose as a gather over grid points: a CSR of L^T holding only node indices, sorted
 //       by (grid point, node) on the device (a radix sort of 64-bit keys), one warp per grid point,
 //       entries in node order, fixed-order lane reduction -- deterministic, no atomics.
@@ -76,29 +76,40 @@ __global__ void low_bits_kernel(const unsigned long long* __restrict__ keys, int
     if (e < count) col[e] = static_cast<int>(keys[e] & 0xffffffffull);
 }
 
-// out[f][node] = sum_taps (wx wy wz) field[f][tap], one warp per node.
-__global__ void interpolate_kernel(const int* __restrict__ base, const double* __restrict__ w1d, int64_t m, int ny,
-                                   int nz, const double* __restrict__ fields, int nf, int64_t field_stride,
-                                   double* __restrict__ out, int64_t out_stride) {
-    // fields are processed five at a time, chunk blockIdx.y
-    const int64_t warp = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+// out[f][node] = sum_taps wx (wy wz field[f][tap]), one warp per node and up to NF fields (blockIdx.y:
+// which NF): a lane holds the (y, z) taps (lane / 8, lane mod 8) and (lane / 8 + 4, lane mod 8), so its
+// weights are formed once, all its 16 NF loads are independent, and a load takes 4 whole rows of 8. For points in no particular order; the
+// quadrature's own nodes go by groups of a cell (interpolate_groups_kernel).
+template <int NF>
+__global__ void __launch_bounds__(256) interpolate_kernel(const int* __restrict__ base,
+                                                          const double* __restrict__ w1d, int64_t m, int ny, int nz,
+                                                          const double* __restrict__ fields, int64_t field_stride,
+                                                          double* __restrict__ out, int64_t out_stride) {
+    const int64_t node = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (warp >= m) return;
-    const int64_t node = warp;
-    const int f0 = blockIdx.y * 5;
-    nf = min(5, nf - f0);
-    fields += f0 * field_stride;
-    out += f0 * out_stride;
-    const int bx = base[node * 3 + 0] - HALFD, by = base[node * 3 + 1] - HALFD, bz = base[node * 3 + 2] - HALFD;
+    if (node >= m) return;
+    fields += blockIdx.y * NF * field_stride;
+    out += blockIdx.y * NF * out_stride;
+    const int b = lane >> 3, c = lane & 7;
     const double* w = w1d + node * 24;
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int t = lane; t < 512; t += 32) {
-        const int a = t >> 6, b = (t >> 3) & 7, c = t & 7;
-        const double v = (w[a] * w[8 + b]) * w[16 + c];
-        const int64_t idx = (static_cast<int64_t>(bx + a) * ny + (by + b)) * nz + (bz + c);
-        for (int f = 0; f < nf; ++f) acc[f] += v * fields[f * field_stride + idx];
+    const double w0 = w[8 + b] * w[16 + c], w1 = w[12 + b] * w[16 + c];
+    const int64_t first = (static_cast<int64_t>(base[node * 3] - HALFD) * ny + (base[node * 3 + 1] - HALFD + b)) * nz +
+                          (base[node * 3 + 2] - HALFD + c);
+    const int64_t plane = static_cast<int64_t>(ny) * nz;
+    double acc[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) acc[f] = 0.0;
+#pragma unroll
+    for (int a = 0; a < KTAP; ++a) {
+        const double wx = w[a];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const double* src = fields + f * field_stride + first + a * plane;
+            acc[f] = fma(wx, fma(w1, src[4 * nz], w0 * src[0]), acc[f]);
+        }
     }
-    for (int f = 0; f < nf; ++f) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
         double s = acc[f];
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
@@ -242,9 +253,24 @@ extern "C" int cdftb_quadrature_interpolate_f64(const int* base, const double* w
     (void)nx;
     if (m < 0 || nf < 1 || nf > 5 * 65535 || (m > 0 && (!base || !w1d || !fields || !out))) return CDFTB_ERR_ARGUMENT;
     if (m == 0) return CDFTB_OK;
-    dim3 grid(blocks_for(m * 32, 256), static_cast<unsigned>(ceil_div(nf, 5)));
-    interpolate_kernel<<<grid, 256, 0, as_stream(stream)>>>(base, w1d, m, ny, nz, fields, nf, field_stride, out,
-                                                            out_stride);
+    cudaStream_t s = as_stream(stream);
+    const unsigned blocks = blocks_for(m * 32, 256);
+    while (nf >= 4) {
+        const int fours = nf / 4 < 65535 ? nf / 4 : 65535;
+        interpolate_kernel<4><<<dim3(blocks, static_cast<unsigned>(fours)), 256, 0, s>>>(
+            base, w1d, m, ny, nz, fields, field_stride, out, out_stride);
+        const int st = check_launch();
+        if (st != CDFTB_OK) return st;
+        fields += int64_t(4) * fours * field_stride;
+        out += int64_t(4) * fours * out_stride;
+        nf -= 4 * fours;
+    }
+    switch (nf) {
+        case 0: return CDFTB_OK;
+        case 1: interpolate_kernel<1><<<blocks, 256, 0, s>>>(base, w1d, m, ny, nz, fields, field_stride, out, out_stride); break;
+        case 2: interpolate_kernel<2><<<blocks, 256, 0, s>>>(base, w1d, m, ny, nz, fields, field_stride, out, out_stride); break;
+        default: interpolate_kernel<3><<<blocks, 256, 0, s>>>(base, w1d, m, ny, nz, fields, field_stride, out, out_stride); break;
+    }
     return check_launch();
 }
 
@@ -401,6 +427,83 @@ __global__ void __launch_bounds__(256, 2) interpolate_grouped_kernel(const int* 
     }
 }
 
+// The interpolant of a few fields over the same groups, one warp per group: lanes hold the (y, z) taps
+// as in interpolate_kernel, each loaded value serves the group's four nodes, and the sums over the lanes
+// halve the values held at every step. Latency bounds it (a group's nodes, cell, weights and box are read
+// one after the other). He 65^3, two fields: 23 us; a warp per node with 16 strided taps per lane took 57 us.
+template <int NF>
+__global__ void __launch_bounds__(256) interpolate_groups_kernel(const int* __restrict__ base,
+                                                                 const double* __restrict__ w1d,
+                                                                 const int* __restrict__ group_nodes,
+                                                                 const int* __restrict__ group_ptr, int64_t groups,
+                                                                 int ny, int nz, const double* __restrict__ fields,
+                                                                 int64_t field_stride, double* __restrict__ out,
+                                                                 int64_t out_stride) {
+    __shared__ double wx[8][GROUP_BATCH][KTAP];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t g = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (g >= groups) return;
+    fields += blockIdx.y * NF * field_stride;
+    out += blockIdx.y * NF * out_stride;
+    const int first = group_ptr[g], last = group_ptr[g + 1];
+    const int lead = group_nodes[first];
+    const int b = lane >> 3, c = lane & 7;
+    const int64_t corner = (static_cast<int64_t>(base[lead * 3] - HALFD) * ny + (base[lead * 3 + 1] - HALFD + b)) * nz +
+                           (base[lead * 3 + 2] - HALFD + c);
+    const int64_t plane = static_cast<int64_t>(ny) * nz;
+    for (int b0 = first; b0 < last; b0 += GROUP_BATCH) {
+        const int count = min(GROUP_BATCH, last - b0);
+        // lane 8 j + a: the x weight a of node j (a short batch repeats its first node)
+        const int own = lane >> 3;
+        const int own_node = group_nodes[b0 + (own < count ? own : 0)];
+        __syncwarp();
+        wx[warp][own][lane & 7] = w1d[int64_t(own_node) * 24 + (lane & 7)];
+        double w0[GROUP_BATCH], w1[GROUP_BATCH];
+#pragma unroll
+        for (int j = 0; j < GROUP_BATCH; ++j) {
+            const double* w = w1d + int64_t(__shfl_sync(0xffffffffu, own_node, 8 * j)) * 24;
+            w0[j] = w[8 + b] * w[16 + c];
+            w1[j] = w[12 + b] * w[16 + c];
+        }
+        __syncwarp();
+        constexpr int V = NF == 1 ? 4 : (NF == 2 ? 8 : 16);  // values to sum, node-major, a power of two
+        double acc[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[k] = 0.0;
+#pragma unroll
+        for (int a = 0; a < KTAP; ++a) {
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                const double* src = fields + f * field_stride + corner + a * plane;
+                const double v0 = src[0], v1 = src[4 * nz];
+#pragma unroll
+                for (int j = 0; j < GROUP_BATCH; ++j)
+                    acc[j * (V / 4) + f] = fma(wx[warp][j][a], fma(w1[j], v1, w0[j] * v0), acc[j * (V / 4) + f]);
+            }
+        }
+        // lane l ends with the sum of value l / (32 / V)
+        int width = V;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            if (width > 1) {
+                width >>= 1;
+                const bool upper = (lane & off) != 0;
+#pragma unroll
+                for (int k = 0; k < V / 2; ++k) {
+                    if (k >= width) break;
+                    const double send = upper ? acc[k] : acc[k + width];
+                    const double keep = upper ? acc[k + width] : acc[k];
+                    acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+            } else {
+                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+            }
+        }
+        const int value = lane / (32 / V), j = value / (V / 4), f = value % (V / 4);
+        if (lane % (32 / V) == 0 && j < count && f < NF) out[f * out_stride + group_nodes[b0 + j]] = acc[0];
+    }
+}
+
 int fields_to_rows(const double* src, int nf, int64_t stride, int64_t n, double* dst, cudaStream_t s) {
     fields_to_rows_kernel<<<static_cast<unsigned>(ceil_div(n, MANY)), dim3(MANY, 8), 0, s>>>(src, nf, stride, n, dst);
     return check_launch();
@@ -466,6 +569,40 @@ extern "C" int cdftb_quadrature_interpolate_grouped_f64(const int* base, const d
         if (st != CDFTB_OK) return st;
     }
     return CDFTB_OK;
+}
+
+extern "C" int cdftb_quadrature_interpolate_groups_f64(const int* base, const double* w1d, int64_t m, int nx, int ny,
+                                                       int nz, const int* group_nodes, const int* group_ptr,
+                                                       int64_t groups, const double* fields, int nf,
+                                                       int64_t field_stride, double* out, int64_t out_stride,
+                                                       cdftb_stream_t stream) {
+    const int64_t n_points = int64_t(nx) * ny * nz;
+    if (m < 0 || nf < 1 || n_points <= 0 || groups < 0 || groups > m ||
+        (m > 0 && (!base || !w1d || !group_nodes || !group_ptr || !fields || !out)))
+        return CDFTB_ERR_ARGUMENT;
+    if (m == 0 || groups == 0) return CDFTB_OK;
+    cudaStream_t s = as_stream(stream);
+    const unsigned blocks = blocks_for(groups * 32, 256);
+#define CDFTB_GROUPS(NF_, CHUNKS_)                                                                        \
+    cdftb::interpolate_groups_kernel<NF_><<<dim3(blocks, static_cast<unsigned>(CHUNKS_)), 256, 0, s>>>(   \
+        base, w1d, group_nodes, group_ptr, groups, ny, nz, fields, field_stride, out, out_stride)
+    while (nf >= 4) {
+        const int fours = nf / 4 < 65535 ? nf / 4 : 65535;
+        CDFTB_GROUPS(4, fours);
+        const int st = check_launch();
+        if (st != CDFTB_OK) return st;
+        fields += int64_t(4) * fours * field_stride;
+        out += int64_t(4) * fours * out_stride;
+        nf -= 4 * fours;
+    }
+    switch (nf) {
+        case 0: return CDFTB_OK;
+        case 1: CDFTB_GROUPS(1, 1); break;
+        case 2: CDFTB_GROUPS(2, 1); break;
+        default: CDFTB_GROUPS(3, 1); break;
+    }
+#undef CDFTB_GROUPS
+    return check_launch();
 }
 
 // The weight of every CSR entry of L^T (the same product as the lift kernels form on the fly).

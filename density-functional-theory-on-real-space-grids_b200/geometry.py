@@ -398,8 +398,9 @@ class CuspQuadrature:
                  *self.grid.shape, ptr(self.group_nodes), ptr(self.group_ptr), self.n_groups, ptr(fields), nf, n,
                  ptr(out), self.n_nodes, ptr(scratch), scratch.numel(), stream_handle(fields.device))
             return out
-        call("cdftb_quadrature_interpolate_f64", ptr(self.base), ptr(self.w1d), self.n_nodes, *self.grid.shape,
-             ptr(fields), nf, n, ptr(out), self.n_nodes, stream_handle(fields.device))
+        call("cdftb_quadrature_interpolate_groups_f64", ptr(self.base), ptr(self.w1d), self.n_nodes, *self.grid.shape,
+             ptr(self.group_nodes), ptr(self.group_ptr), self.n_groups, ptr(fields), nf, n, ptr(out), self.n_nodes,
+             stream_handle(fields.device))
         return out
 
     def _lift_raw(self, x: torch.Tensor, nf: int) -> torch.Tensor:

@@ -138,9 +138,7 @@ class KohnShamStep:
         call("cdftb_hartree_split_f64", ptr(n_grid), ptr(self._f2_grid), ptr(g.step.cusp_grid), ptr(coef), na, n, 1,
              ptr(rho), ptr(n_smooth), stream)
         self.poisson.solve_batch(n_smooth.reshape(1, n), out=fields[1].reshape(1, n))
-        node_fields = torch.empty((2, m), dtype=torch.float64, device=dev)
-        call("cdftb_quadrature_interpolate_f64", ptr(q.base), ptr(q.w1d), m, *grid.shape, ptr(fields), 2, n,
-             ptr(node_fields), m, stream)
+        node_fields = q._interp_raw(fields, 2)
         lift_in = torch.empty((2, m), dtype=torch.float64, device=dev)
         e_w = torch.empty(m, dtype=torch.float64, device=dev)
         call("cdftb_potentials_node_lda_f64", ptr(node_fields), m, ptr(q.weights), ptr(q.f2), ptr(g.step.v1s_node),

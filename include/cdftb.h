@@ -359,6 +359,12 @@ int cdftb_quadrature_interpolate_grouped_f64(const int* base, const double* w1d,
                                              const double* fields, int nf, int64_t field_stride, double* out,
                                              int64_t out_stride, void* scratch, int64_t scratch_bytes,
                                              cdftb_stream_t stream);
+/* The interpolant of a few fields over the same groups, without scratch: equals
+ * cdftb_quadrature_interpolate_f64 up to the order of the sums (~1e-16 relative). */
+int cdftb_quadrature_interpolate_groups_f64(const int* base, const double* w1d, int64_t m, int nx, int ny, int nz,
+                                            const int* group_nodes, const int* group_ptr, int64_t groups,
+                                            const double* fields, int nf, int64_t field_stride, double* out,
+                                            int64_t out_stride, cdftb_stream_t stream);
 int cdftb_quadrature_lift_many_f64(const long long* row_ptr, const int* col, const double* values, const int* seg_ptr,
                                    const int* seg_row, int64_t seg_capacity, int nx, int ny, int nz, int64_t m,
                                    const double* node_values, int nf, int64_t x_stride, double* out,

@@ -1,4 +1,4 @@
-"""L and L^T over nodes sorted by base cell, against the entry points over the list of entries."""
+"""L and L^T over nodes sorted by base cell, against the entry points over the list of entries and over single nodes."""
 
 from __future__ import annotations
 
@@ -67,3 +67,22 @@ def test_lift_takes_strided_rows(pkg, quadrature, nf):
                   torch.cuda.current_stream().cuda_stream)
     assert torch.equal(out[:, :n], q._lift_raw(x[:, :m].contiguous(), nf))
     assert bool((out[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("nf", [1, 2, 3, 4, 5, 6, 7])
+def test_interpolant_of_a_few_fields(pkg, quadrature, nf):
+    """Groups of a cell against a warp per node and the many-field kernel: 512 products of sums of weights
+    below 3 per axis, 1e-13 of the largest value."""
+    q = quadrature
+    n, m = q.grid.n_points, q.n_nodes
+    g = torch.Generator().manual_seed(nf)
+    fields = torch.randn((nf, n), dtype=torch.float64, generator=g).cuda()
+    got = q._interp_raw(fields, nf)
+    one = torch.full((nf, m + 3), 7.0, dtype=torch.float64, device="cuda:0")
+    pkg._lib.call("cdftb_quadrature_interpolate_f64", q.base.data_ptr(), q.w1d.data_ptr(), m, *q.grid.shape,
+                  fields.data_ptr(), nf, n, one.data_ptr(), m + 3, torch.cuda.current_stream().cuda_stream)
+    many = q._interp_raw(fields.repeat(8, 1), 8 * nf)[:nf]
+    scale = float(many.abs().max())
+    torch.testing.assert_close(got, many, rtol=0, atol=1e-13 * scale)
+    torch.testing.assert_close(one[:, :m], many, rtol=0, atol=1e-13 * scale)
+    assert bool((one[:, m:] == 7.0).all())
