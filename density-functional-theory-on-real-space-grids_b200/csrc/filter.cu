@@ -729,7 +729,7 @@ struct WideShape {
     static constexpr int T = WARPS * 32;
     // odd row pitches (in 16-byte points): the 8 rows of a warp's z items then fall on 8 different
     // groups of 4 banks (an even pitch such as TZ + 18 puts them on 4)
-    static constexpr int BW = TZ + 19;  // phi box: z0-8 .. z0+TZ+10
+    static constexpr int BW = TZ + 15;  // phi box: z0-8 .. z0+TZ+6, the last node of the tile's last z face
     static constexpr int ZROW = TZ + 3;
     static constexpr unsigned TX_PHI = NROWW * BW * EB;
     static constexpr unsigned TX_PREV = TYW * TZ * EB;
@@ -1204,58 +1204,92 @@ __global__ void pack_lanes_kernel(const void* __restrict__ in, int in_dtype, int
     }
 }
 
-// Wide lanes from a caller block: lane l holds orbitals ORB l .. ORB l + ORB - 1 as one 16-byte
-// element per point, padding and missing orbitals zero. blockIdx.y walks the lanes; one point per
-// thread.
-template <typename W>
-__global__ void pack_wide_kernel(const void* __restrict__ in, int in_dtype, int64_t batch, int nx, int ny, int nz,
-                                 int nzp, int64_t lanes, int opg, int lpg, typename W::E* __restrict__ out) {
-    using S = typename W::S;
-    constexpr int ORB = W::ORB;
-    const int64_t per_lane = int64_t(nx) * ny * nzp;
-    const int64_t n_points = int64_t(nx) * ny * nz;
-    const bool narrow = per_lane <= 0xffffffffll;
-    for (int64_t l = blockIdx.y; l < lanes; l += gridDim.y) {
-        typename W::E* dst = out + l * per_lane;
+// What a filter or apply call copies before its first slab launch, in one launch: the geometry and the
+// potentials into rows padded to 16 bytes (for TMA), and the caller's block into wide lanes -- lane l
+// holds orbitals ORB l .. ORB l + ORB - 1 as one 16-byte element per point, padding and missing orbitals
+// zero. A CTA takes kPrepPerBlock elements of one job; the jobs' CTAs follow each other in the grid.
+// HBM bounds it for a batch (5.2 TB/s); for one system it is the launches that cost: five copies and a
+// pack of 2 to 6 us each, 25 us of a 33^3 apply's 39.
+constexpr int kPrepThreads = 256;
+constexpr int kPrepPerBlock = 4 * kPrepThreads;
+
+struct PadJob {
+    const void* src;         // null: zeros
+    void* dst;
+    int64_t total;           // elements written
+    int cols, cols_pad;      // source row -> padded row (zeros behind)
+    int64_t group_rows;      // rows per group and the groups' distance in the source
+    int64_t group_stride;
+    int64_t first_block;
+};
+
+struct PrepArgs {
+    PadJob pad[5];
+    int64_t pack_first;      // the first CTA of the lanes (none: the grid ends there)
+    int64_t lane_blocks;     // CTAs per lane
+    const void* block;
+    int block_dtype;
+    int64_t batch;
+    int nx, ny, nz, nzp;
+    int opg, lpg;
+    void* lanes;
+};
+
+template <typename L>
+__global__ void __launch_bounds__(kPrepThreads) prep_kernel(const __grid_constant__ PrepArgs a) {
+    using S = typename L::S;
+    const int64_t b = blockIdx.x;
+    if (b < a.pack_first) {
+        int j = 0;
+#pragma unroll
+        for (int k = 1; k < 5; ++k) j += b >= a.pad[k].first_block ? 1 : 0;
+        const PadJob job = a.pad[j];
+        const S* src = static_cast<const S*>(job.src);
+        const int64_t base = (b - job.first_block) * kPrepPerBlock + threadIdx.x;
+        const bool narrow = job.total <= 0xffffffffll;
+        S v[kPrepPerBlock / kPrepThreads];
+#pragma unroll
+        for (int u = 0; u < kPrepPerBlock / kPrepThreads; ++u) {
+            const int64_t k = base + u * kPrepThreads;
+            v[u] = S(0);
+            if (k >= job.total || !src) continue;
+            const int64_t row = narrow ? static_cast<unsigned>(k) / static_cast<unsigned>(job.cols_pad) : k / job.cols_pad;
+            const int c = static_cast<int>(k - row * job.cols_pad);
+            if (c >= job.cols) continue;
+            const int64_t g = job.group_rows > row ? 0 : row / job.group_rows;
+            v[u] = src[g * job.group_stride + (row - g * job.group_rows) * job.cols + c];
+        }
+#pragma unroll
+        for (int u = 0; u < kPrepPerBlock / kPrepThreads; ++u)
+            if (const int64_t k = base + u * kPrepThreads; k < job.total) static_cast<S*>(job.dst)[k] = v[u];
+        return;
+    }
+    if constexpr (L::WIDE) {
+        constexpr int ORB = L::ORB;
+        const int64_t per_lane = int64_t(a.nx) * a.ny * a.nzp;
+        const int64_t n_points = int64_t(a.nx) * a.ny * a.nz;
+        const int64_t l = (b - a.pack_first) / a.lane_blocks;
+        const int64_t base = (b - a.pack_first - l * a.lane_blocks) * kPrepPerBlock + threadIdx.x;
+        const bool narrow = per_lane <= 0xffffffffll;
         int64_t orb[ORB];
 #pragma unroll
-        for (int h = 0; h < ORB; ++h) orb[h] = lane_orbital<ORB>(l, h, batch, opg, lpg);
-        for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < per_lane;
-             k += int64_t(gridDim.x) * blockDim.x) {
-            int64_t xy;
-            int zp;
-            if (narrow) {
-                const unsigned uk = static_cast<unsigned>(k), row = uk / static_cast<unsigned>(nzp);
-                xy = row;
-                zp = static_cast<int>(uk - row * static_cast<unsigned>(nzp));
-            } else {
-                xy = k / nzp;
-                zp = static_cast<int>(k - xy * nzp);
-            }
-            S v[ORB];
+        for (int h = 0; h < ORB; ++h) orb[h] = lane_orbital<ORB>(l, h, a.batch, a.opg, a.lpg);
+        typename L::E* dst = static_cast<typename L::E*>(a.lanes) + l * per_lane;
+        S v[kPrepPerBlock / kPrepThreads][ORB];
 #pragma unroll
-            for (int h = 0; h < ORB; ++h) v[h] = S(0);
-            if (zp < nz) {
-                const int64_t pt = xy * nz + zp;
+        for (int u = 0; u < kPrepPerBlock / kPrepThreads; ++u) {
+            const int64_t k = base + u * kPrepThreads;
+            const int64_t xy = narrow ? static_cast<unsigned>(k) / static_cast<unsigned>(a.nzp) : k / a.nzp;
+            const int zp = static_cast<int>(k - xy * a.nzp);
+            const int64_t pt = xy * a.nz + zp;
+            const bool in = k < per_lane && zp < a.nz;
 #pragma unroll
-                for (int h = 0; h < ORB; ++h)
-                    if (orb[h] >= 0) v[h] = load_as<S>(in, in_dtype, orb[h] * n_points + pt);
-            }
-            dst[k] = W::make(v);
+            for (int h = 0; h < ORB; ++h)
+                v[u][h] = in && orb[h] >= 0 ? load_as<S>(a.block, a.block_dtype, orb[h] * n_points + pt) : S(0);
         }
-    }
-}
-
-// rows x cols -> rows x cols_pad (zeros in the padding), for the geometry copies TMA reads.
-template <typename S>
-__global__ void pad_rows_kernel(const S* __restrict__ src, int64_t rows, int cols, int cols_pad, int64_t src_stride,
-                                S* __restrict__ dst) {
-    const int64_t total = rows * cols_pad;
-    for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
-         idx += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t r = idx / cols_pad;
-        const int c = static_cast<int>(idx - r * cols_pad);
-        dst[idx] = c < cols ? src[r * src_stride + c] : S(0);
+#pragma unroll
+        for (int u = 0; u < kPrepPerBlock / kPrepThreads; ++u)
+            if (const int64_t k = base + u * kPrepThreads; k < per_lane) dst[k] = L::make(v[u]);
     }
 }
 
@@ -1414,47 +1448,55 @@ int launch_slab(const FilterMaps& maps, FilterArgs a, int64_t lanes, cudaStream_
     return CDFTB_OK;
 }
 
+// The padded copies at geo_base (element type S), in the order of geo_pack.
 template <typename S>
-int pad_rows(const void* src, int64_t rows, int cols, int cols_pad, S* dst, cudaStream_t stream) {
-    const int64_t total = rows * cols_pad;
-    const unsigned blocks = static_cast<unsigned>(std::min<int64_t>(ceil_div(total, 256), 148 * 16));
-    pad_rows_kernel<S><<<blocks, 256, 0, stream>>>(static_cast<const S*>(src), rows, cols, cols_pad, cols, dst);
-    return check_launch();
-}
+struct GeoCopies {
+    S *w0, *w1, *w2, *inv, *pot;
+    GeoCopies(const GeoPack& gp, void* geo_base) {
+        w0 = static_cast<S*>(geo_base);
+        w1 = w0 + gp.n_w0;
+        w2 = w1 + gp.n_w1;
+        inv = w2 + gp.n_w2;
+        pot = inv + gp.n_inv;
+    }
+};
 
-// Copies the geometry into the padded rows TMA reads (at geo, element type S) and encodes the maps
-// of the geometry; kinetic_only zeroes the potential rows instead of copying them.
+// The jobs that copy the geometry into the padded rows TMA reads; without_potential zeroes the
+// potential rows instead of copying them. Returns the CTAs they take.
 template <typename Lane>
-int prepare_geometry(const cdftb_operator* op, int64_t batch, void* geo_base, int ty, int tz, bool kinetic_only,
-                     FilterMaps* maps, cudaStream_t stream) {
+int64_t geometry_jobs(const cdftb_operator* op, int64_t batch, void* geo_base, bool without_potential, PrepArgs* args) {
     using S = typename Lane::S;
-    const int nx = op->nx, ny = op->ny, nz = op->nz;
+    const int64_t nx = op->nx, ny = op->ny, nz = op->nz;
     const GeoPack gp = geo_pack(op, batch);
-    S* w0p = static_cast<S*>(geo_base);
-    S* w1p = w0p + gp.n_w0;
-    S* w2p = w1p + gp.n_w1;
-    S* invp = w2p + gp.n_w2;
-    S* potp = invp + gp.n_inv;
+    const GeoCopies<S> to(gp, geo_base);
     const int64_t nsys = systems_of(op, batch);
     const int64_t ng = geometry_systems(op, batch);  // per-system arrays follow each other in memory
-    int st;
-    if ((st = pad_rows<S>(op->face_weights[0], ng * (nx + 8) * ny, nz, gp.nzg, w0p, stream)) != CDFTB_OK) return st;
-    if ((st = pad_rows<S>(op->face_weights[1], ng * nx * (ny + 8), nz, gp.nzg, w1p, stream)) != CDFTB_OK) return st;
-    if ((st = pad_rows<S>(op->face_weights[2], ng * nx * ny, nz + 8, gp.nz8g, w2p, stream)) != CDFTB_OK) return st;
-    if ((st = pad_rows<S>(op->inverse_weight, ng * nx * ny, nz, gp.nzg, invp, stream)) != CDFTB_OK) return st;
-    if (kinetic_only || !op->potential) {
-        if ((st = check(cudaMemsetAsync(potp, 0, gp.n_pot * sizeof(S), stream))) != CDFTB_OK) return st;
-    } else if (op->potential_stride == 0 || op->potential_stride == int64_t(nx) * ny * nz) {
-        // every system's row block at once (rows of consecutive systems are consecutive)
-        if ((st = pad_rows<S>(op->potential, nsys * nx * ny, nz, gp.nzg, potp, stream)) != CDFTB_OK) return st;
-    } else {
-        for (int64_t g = 0; g < nsys; ++g) {
-            const void* src = static_cast<const S*>(op->potential) + g * op->potential_stride;
-            if ((st = pad_rows<S>(src, int64_t(nx) * ny, nz, gp.nzg, potp + g * int64_t(nx) * ny * gp.nzg, stream)) !=
-                CDFTB_OK)
-                return st;
-        }
-    }
+    int64_t blocks = 0;
+    auto job = [&](int i, const void* src, void* dst, int64_t rows, int64_t cols, int cols_pad, int64_t group_rows,
+                   int64_t group_stride) {
+        args->pad[i] = PadJob{src, dst, rows * cols_pad, static_cast<int>(cols), cols_pad, group_rows, group_stride, blocks};
+        blocks += ceil_div(rows * cols_pad, kPrepPerBlock);
+    };
+    auto whole = [&](int i, const void* src, void* dst, int64_t rows, int64_t cols, int cols_pad) {
+        job(i, src, dst, rows, cols, cols_pad, rows + 1, 0);
+    };
+    whole(0, op->face_weights[0], to.w0, ng * (nx + 8) * ny, nz, gp.nzg);
+    whole(1, op->face_weights[1], to.w1, ng * nx * (ny + 8), nz, gp.nzg);
+    whole(2, op->face_weights[2], to.w2, ng * nx * ny, nz + 8, gp.nz8g);
+    whole(3, op->inverse_weight, to.inv, ng * nx * ny, nz, gp.nzg);
+    job(4, without_potential ? nullptr : op->potential, to.pot, nsys * nx * ny, nz, gp.nzg, nx * ny, op->potential_stride);
+    return blocks;
+}
+
+// The maps of the padded geometry at geo_base, for tiles of ty x tz.
+template <typename Lane>
+int encode_geometry(const cdftb_operator* op, int64_t batch, void* geo_base, int ty, int tz, FilterMaps* maps) {
+    using S = typename Lane::S;
+    const int nx = op->nx, ny = op->ny;
+    const GeoPack gp = geo_pack(op, batch);
+    const GeoCopies<S> at(gp, geo_base);
+    const int64_t nsys = systems_of(op, batch);
+    const int64_t ng = geometry_systems(op, batch);
     const CUtensorMapDataType gt = Lane::GEO_TYPE;
     const int sb = sizeof(S);
     const unsigned tile_box[4] = {unsigned(tz), unsigned(ty), 1, 1};
@@ -1465,12 +1507,12 @@ int prepare_geometry(const cdftb_operator* op, int64_t batch, void* geo_base, in
     const unsigned b_w2[4] = {unsigned(tz + 8), unsigned(ty), 1, 1};
     const int64_t d_inv[4] = {gp.nzg, ny, nx, ng};
     const int64_t d_pot[4] = {gp.nzg, ny, nx, nsys};
-    const unsigned b_pot[4] = {unsigned(tz), unsigned(ty), 1, 1};
-    if ((st = encode_map(&maps->w0, gt, sb, 4, w0p, d_w0, tile_box)) != CDFTB_OK) return st;
-    if ((st = encode_map(&maps->w1, gt, sb, 4, w1p, d_w1, b_w1)) != CDFTB_OK) return st;
-    if ((st = encode_map(&maps->w2, gt, sb, 4, w2p, d_w2, b_w2)) != CDFTB_OK) return st;
-    if ((st = encode_map(&maps->inv, gt, sb, 4, invp, d_inv, tile_box)) != CDFTB_OK) return st;
-    return encode_map(&maps->pot, gt, sb, 4, potp, d_pot, b_pot);
+    int st;
+    if ((st = encode_map(&maps->w0, gt, sb, 4, at.w0, d_w0, tile_box)) != CDFTB_OK) return st;
+    if ((st = encode_map(&maps->w1, gt, sb, 4, at.w1, d_w1, b_w1)) != CDFTB_OK) return st;
+    if ((st = encode_map(&maps->w2, gt, sb, 4, at.w2, d_w2, b_w2)) != CDFTB_OK) return st;
+    if ((st = encode_map(&maps->inv, gt, sb, 4, at.inv, d_inv, tile_box)) != CDFTB_OK) return st;
+    return encode_map(&maps->pot, gt, sb, 4, at.pot, d_pot, tile_box);
 }
 
 template <typename Lane>
@@ -1577,24 +1619,11 @@ int launch_wide(const FilterMaps& maps, const FilterArgs& a, int64_t lanes, cuda
 int encode_wide_lane_maps(void* buf, int nzp, int ny, int nx, int64_t lanes, int ty, int tz, CUtensorMap* phi,
                           CUtensorMap* prev) {
     const int64_t lane_dims[4] = {2 * int64_t(nzp), ny, nx, lanes};
-    const unsigned phi_box[4] = {unsigned(2 * (tz + 19)), unsigned(ty + 2 * HALO), 1, 1};  // WideShape::BW points
+    const unsigned phi_box[4] = {unsigned(2 * (tz + 15)), unsigned(ty + 2 * HALO), 1, 1};  // WideShape::BW points
     const unsigned prev_box[4] = {unsigned(2 * tz), unsigned(ty), 1, 1};
     int st = encode_map(phi, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, 4, buf, lane_dims, phi_box);
     if (st == CDFTB_OK) st = encode_map(prev, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, 4, buf, lane_dims, prev_box);
     return st;
-}
-
-template <typename W>
-int pack_wide(const void* block, int in_dtype, int64_t batch, int nx, int ny, int nz, int nzp, int64_t lanes,
-              int opg, int lpg, void* dst, cudaStream_t stream) {
-    if ((reinterpret_cast<uintptr_t>(dst) & 15) != 0) return CDFTB_ERR_ARGUMENT;
-    const int64_t per_lane = int64_t(nx) * ny * nzp;
-    const unsigned ly = static_cast<unsigned>(std::min<int64_t>(lanes, 65535));
-    const unsigned bx = static_cast<unsigned>(
-        std::max<int64_t>(1, std::min<int64_t>(ceil_div(per_lane, 256), ceil_div(int64_t(148) * 16, ly))));
-    pack_wide_kernel<W><<<dim3(bx, ly), 256, 0, stream>>>(block, in_dtype, batch, nx, ny, nz, nzp, lanes, opg, lpg,
-                                                          static_cast<typename W::E*>(dst));
-    return check_launch();
 }
 
 // The same steps for both lane layouts: two-orbital (LaneF2) or one-orbital (LaneD) lane points of
@@ -1636,14 +1665,35 @@ int encode_lanes(void* buf, int nzp, int ny, int nx, int64_t lanes, int ty, int 
         return encode_lane_maps(buf, nzp, ny, nx, lanes, tz, phi, prev);
 }
 
+// The call's copies: the caller's block into lanes at dst, the geometry into padded rows at geo_base.
 template <typename L>
-int pack_lanes(const cdftb_operator* op, const void* block, int in_dtype, int64_t batch, int nx, int ny, int nz,
-               int nzp, int64_t lanes, void* dst, cudaStream_t stream) {
-    if constexpr (L::WIDE)
-        return pack_wide<L>(block, in_dtype, batch, nx, ny, nz, nzp, lanes, op->orbitals_per_group,
-                            wide_lanes_per_group(op, L::ORB), dst, stream);
-    else
-        return pack_block<L>(op, block, in_dtype, batch, nx, ny, nz, nzp, lanes, dst, stream);
+int prepare(const cdftb_operator* op, const void* block, int in_dtype, int64_t batch, int64_t lanes, void* dst,
+            void* geo_base, bool without_potential, cudaStream_t stream) {
+    if ((reinterpret_cast<uintptr_t>(dst) & 15) != 0) return CDFTB_ERR_ARGUMENT;
+    PrepArgs a{};
+    int64_t blocks = geometry_jobs<L>(op, batch, geo_base, without_potential || !op->potential, &a);
+    a.pack_first = blocks;
+    const int nzp = padded_z(op->nz);
+    if constexpr (L::WIDE) {
+        a.lane_blocks = ceil_div(int64_t(op->nx) * op->ny * nzp, kPrepPerBlock);
+        a.block = block;
+        a.block_dtype = in_dtype;
+        a.batch = batch;
+        a.nx = op->nx;
+        a.ny = op->ny;
+        a.nz = op->nz;
+        a.nzp = nzp;
+        a.opg = op->orbitals_per_group;
+        a.lpg = wide_lanes_per_group(op, L::ORB);
+        a.lanes = dst;
+        blocks += lanes * a.lane_blocks;
+    } else {
+        const int st = pack_block<L>(op, block, in_dtype, batch, op->nx, op->ny, op->nz, nzp, lanes, dst, stream);
+        if (st != CDFTB_OK) return st;
+    }
+    if (blocks > 0x7fffffffll) return CDFTB_ERR_CAPACITY;
+    prep_kernel<L><<<static_cast<unsigned>(blocks), kPrepThreads, 0, stream>>>(a);
+    return check_launch();
 }
 
 // The tilings (rows TY x columns TZ) each lane layout has: the 8-byte-lane kernel 8 x 32 and 8 x 36;
@@ -1718,7 +1768,7 @@ bool tuned_choice(const TuneKey& key, TileChoice* out) {
     return true;
 }
 
-// Times every candidate tiling: one untimed launch, then three timed ones each. With apply null,
+// Times every candidate tiling (the geometry's padded rows are in place): one untimed launch, then three timed ones each. With apply null,
 // the launch is the first Chebyshev step (packed block in buf[2] -> buf[0]); otherwise it is the
 // apply described by *apply (packed block in buf[2], written to the caller's output, which the
 // real launch then rewrites). Synchronises the stream.
@@ -1742,8 +1792,7 @@ int tune_slab(const cdftb_operator* op, int64_t batch, void* geo_base, void* buf
     for (int ti = 0; ti < count; ++ti) {
         const int ty = list[ti].ty, tz = list[ti].tz;
         FilterMaps m{};
-        const bool kinetic = apply != nullptr && apply->kinetic_only;
-        if ((st = prepare_geometry<Lane>(op, batch, geo_base, ty, tz, kinetic, &m, stream)) != CDFTB_OK) break;
+        if ((st = encode_geometry<Lane>(op, batch, geo_base, ty, tz, &m)) != CDFTB_OK) break;
         if ((st = encode_lanes<Lane>(buf[2], nzp, ny, nx, lanes, ty, tz, &m.phi, &m.prev)) != CDFTB_OK) break;
         FilterArgs a = lane_args<Lane>(op, batch);
         if (apply) {
@@ -1794,7 +1843,7 @@ int slab_filter(const cdftb_operator* op, const void* block, int in_dtype, void*
     const int64_t lane_bytes = int64_t(nx) * ny * nzp * lane_point_bytes<Lane>();
     char* w = static_cast<char*>(work);
     void* buf[3] = {w, w + lanes * lane_bytes, w + 2 * lanes * lane_bytes};
-    int st = pack_lanes<Lane>(op, block, in_dtype, batch, nx, ny, nz, nzp, lanes, buf[2], stream);
+    int st = prepare<Lane>(op, block, in_dtype, batch, lanes, buf[2], w + 3 * lanes * lane_bytes, false, stream);
     if (st != CDFTB_OK) return st;
     const Tile t0 = choose_tile<Lane>(ny, nzp);
     TileChoice choice{t0.ty, t0.tz, 0};
@@ -1813,9 +1862,7 @@ int slab_filter(const cdftb_operator* op, const void* block, int in_dtype, void*
     }
     const int ty = choice.ty, tz = choice.tz;
     FilterMaps geo_maps{};
-    if ((st = prepare_geometry<Lane>(op, batch, w + 3 * lanes * lane_bytes, ty, tz, false, &geo_maps, stream)) !=
-        CDFTB_OK)
-        return st;
+    if ((st = encode_geometry<Lane>(op, batch, w + 3 * lanes * lane_bytes, ty, tz, &geo_maps)) != CDFTB_OK) return st;
     FilterMaps maps[3];
     for (int b = 0; b < 3; ++b)
         if ((st = encode_lanes<Lane>(buf[b], nzp, ny, nx, lanes, ty, tz, &maps[b].phi, &maps[b].prev)) != CDFTB_OK)
@@ -1855,7 +1902,7 @@ int slab_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* ou
     TileChoice choice{t0.ty, t0.tz, 0};
     const TuneKey key = tune_key(op, lanes, Lane::WIDE);
     const bool known = tuned_choice(key, &choice);
-    int st = pack_lanes<Lane>(op, phi, in_dtype, batch, nx, ny, nz, nzp, lanes, w, stream);
+    int st = prepare<Lane>(op, phi, in_dtype, batch, lanes, w, w + lanes * lane_bytes, kinetic_only != 0, stream);
     if (st != CDFTB_OK) return st;
     bool autotune;
     {
@@ -1879,9 +1926,7 @@ int slab_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* ou
     }
     const int ty = choice.ty, tz = choice.tz;
     FilterMaps m{};
-    if ((st = prepare_geometry<Lane>(op, batch, w + lanes * lane_bytes, ty, tz, kinetic_only != 0, &m, stream)) !=
-        CDFTB_OK)
-        return st;
+    if ((st = encode_geometry<Lane>(op, batch, w + lanes * lane_bytes, ty, tz, &m)) != CDFTB_OK) return st;
     if ((st = encode_lanes<Lane>(w, nzp, ny, nx, lanes, ty, tz, &m.phi, &m.prev)) != CDFTB_OK) return st;
     FilterArgs a = lane_args<Lane>(op, batch);
     a.apply_only = 1;
