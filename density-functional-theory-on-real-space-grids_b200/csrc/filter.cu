@@ -37,6 +37,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -712,9 +713,8 @@ struct WideD2 {  // two float64 orbitals
     }
 };
 
-// Plane slots of the wide kernel (16-byte elements: a slot is 31-41 KB): as many as shared memory
-// holds beside a result ring of at least 4, up to kWideMaxSlots. A deeper ring keeps more copies in
-// flight per SM, which is what hides the copies' latency behind the march.
+// Plane slots of the wide kernel (16-byte elements: a slot is 31-41 KB): as many pairs as shared memory
+// holds beside a result ring of at least 4, up to kWideMaxSlots.
 constexpr int kWideMaxSlots = 6;
 constexpr size_t kWideSmem = 232448;  // the opt-in shared memory of one CTA
 
@@ -730,6 +730,9 @@ struct WideShape {
     static constexpr int NZS = (TZ + TYW - 1) / TYW;
     static constexpr int ITEMS = TZ + TYW * NZS;
     static constexpr int PWG = (ITEMS + 31) / 32;
+    // warps of y items only and z items only, where that takes no more warps than mixing them
+    static constexpr int YU = (TZ + 31) / 32, ZU = (TYW * NZS + 31) / 32;
+    static constexpr bool SPLIT = ORB == 4 && YU + ZU == PWG;
     static constexpr int PW = NG * PWG;
     static constexpr int WARPS = MW + PW + 1;
     static constexpr int T = WARPS * 32;
@@ -758,7 +761,7 @@ struct WideShape {
     static constexpr size_t need(int rw, int ry) { return rw * SLOT + ry * YZ_SLOT + (2 * rw + 2 * ry) * 8; }
     static constexpr int slots() {
         int rw = kWideMaxSlots;
-        while (rw > 2 && need(rw, 4) > kWideSmem) --rw;
+        while (rw > NG && need(rw, 4) > kWideSmem) rw -= NG;
         return rw;
     }
     static constexpr int RWS = slots();
@@ -773,7 +776,12 @@ struct WideShape {
     static constexpr size_t O_YZ = RWS * SLOT;
     static constexpr size_t O_BAR = O_YZ + RYW * YZ_SLOT;
     static constexpr size_t BYTES = O_BAR + (2 * RWS + 2 * RYW) * 8;
-    static_assert(RWS >= NG && need(RWS, RYW) <= kWideSmem, "the rings fit one CTA's shared memory");
+    static_assert(need(RWS, RYW) <= kWideSmem, "the rings fit one CTA's shared memory");
+    // A slot is always served by the same pass group. A barrier's parity tells a phase from the next one
+    // only, and a group takes every other plane: with an odd ring it could ask for a plane's copies before
+    // those of the slot's previous plane, which it does not wait for, had landed (copies need not land in
+    // order), and take the answer for its own.
+    static_assert(RWS % NG == 0, "a slot is always served by the same pass group");
     static_assert(TZ >= TYW && TZ % 4 == 0, "z segments of TYW inside the tile; 16-byte float32 geometry rows");
     static_assert(BW % 2 == 1 && ZROW % 2 == 1, "odd row pitches");
     static_assert((TZ - TYW) + NROWW <= BW - 1, "the last z segment's nodes lie inside the phi box");
@@ -782,6 +790,34 @@ struct WideShape {
     static_assert(TYW * TZ >= 32, "a tile of at least one warp");
     static_assert(BYTES <= 232448, "fits the opt-in shared memory of one CTA");
 };
+
+// A pass item: the TYW outputs of a line segment from its TYW + 14 nodes (stride ns) and TYW + 7 face
+// weights (stride ws), streamed through a window of 8 nodes.
+template <typename W, int TYW, typename NS, typename WS>
+__device__ __forceinline__ void pass_item(const typename W::E* nodes, NS ns, const typename W::S* w, WS ws,
+                                          const typename W::T (&tap4)[4], typename W::E (&acc)[TYW]) {
+    typename W::E win[8];
+#pragma unroll
+    for (int r = 0; r < TYW + 2 * HALO; ++r) {
+        win[r & 7] = nodes[r * ns];
+        if (r >= 7) {
+            const int rf = r - 7;  // face rf from nodes rf .. rf + 7
+            // the taps are antisymmetric (tap[7 - j] = -tap[j]): four independent
+            // differences, then a chain of four (depth 5 instead of 8)
+            typename W::E sum = W::mult(tap4[0], W::sub(win[rf & 7], win[(rf + 7) & 7]));
+#pragma unroll
+            for (int j = 1; j < 4; ++j)
+                sum = W::fmat(tap4[j], W::sub(win[(rf + j) & 7], win[(rf + 7 - j) & 7]), sum);
+            const typename W::E f = W::mult(W::splat(w[rf * ws]), sum);
+            // face rf reaches outputs o = rf - 7 .. rf with tap o + 7 - rf
+#pragma unroll
+            for (int o = 0; o < TYW; ++o) {
+                if (o < rf - 7 || o > rf) continue;
+                acc[o] = (o == rf) ? W::mult_neg(tap4[0], f) : W::fmat_k(tap4, o + 7 - rf, f, acc[o]);
+            }
+        }
+    }
+}
 
 // One CTA per SM: the register budget per thread. The SM's 64 K registers are four files of 16 K,
 // one per scheduler, and a CTA's warps are spread over the four, so the scheduler with the most
@@ -803,7 +839,6 @@ __global__ void __maxnreg__((wide_max_registers<WideShape<TYW, TZ, sizeof(typena
     constexpr int ORB = W::ORB;
     using SH = WideShape<TYW, TZ, sizeof(S), ORB>;
     constexpr int TY = TYW;              // this kernel's tile rows (the 8-byte-lane kernel keeps 8)
-    constexpr int NROW = SH::NROWW;
     constexpr int BW = SH::BW;
     extern __shared__ __align__(1024) unsigned char smem[];
     const unsigned bar_full = smem_u32(smem + SH::O_BAR);
@@ -946,68 +981,103 @@ __global__ void __maxnreg__((wide_max_registers<WideShape<TYW, TZ, sizeof(typena
     }
 
     if (warp >= SH::MW) {
-        // ------------------------------------------------------------------ pass groups
         const int pg = (warp - SH::MW) / SH::PWG;
-        const int it = t - (SH::MW + pg * SH::PWG) * 32;
-        bool active = false;
-        int nb = 0, ns = 0, wb = 0, ws = 0, ob = 0, os = 0, first = 0;
-        if (it < TZ) {
-            const int zc = it;
-            active = z0 + zc < nz;
-            nb = zc + 8;
-            ns = BW;
-            wb = SH::O_W1 / sizeof(S) + zc;
-            ws = TZ;
-            ob = zc;
-            os = TZ;
-        } else if (it < SH::ITEMS) {
-            const int zi = it - TZ;
-            const int ry = zi % TY;
-            const int seg = zi / TY;
-            const int zs = min(seg * TY, TZ - TY);
-            first = seg * TY - zs;
-            active = y0 + ry < ny && z0 + zs < nz;
-            nb = (ry + HALO) * BW + zs + 1;
-            ns = 1;
-            wb = SH::O_W2 / sizeof(S) + ry * (TZ + 8) + zs;
-            ws = 1;
-            ob = int(SH::YZ_Z / sizeof(E)) + ry * SH::ZROW + zs;
-            os = 1;
+        if constexpr (!SH::SPLIT) {
+            const int it = t - (SH::MW + pg * SH::PWG) * 32;
+            bool active = false;
+            int nb = 0, ns = 0, wb = 0, ws = 0, ob = 0, os = 0, first = 0;
+            if (it < TZ) {
+                const int zc = it;
+                active = z0 + zc < nz;
+                nb = zc + 8;
+                ns = BW;
+                wb = SH::O_W1 / sizeof(S) + zc;
+                ws = TZ;
+                ob = zc;
+                os = TZ;
+            } else if (it < SH::ITEMS) {
+                const int zi = it - TZ;
+                const int ry = zi % TY;
+                const int seg = zi / TY;
+                const int zs = min(seg * TY, TZ - TY);
+                first = seg * TY - zs;
+                active = y0 + ry < ny && z0 + zs < nz;
+                nb = (ry + HALO) * BW + zs + 1;
+                ns = 1;
+                wb = SH::O_W2 / sizeof(S) + ry * (TZ + 8) + zs;
+                ws = 1;
+                ob = int(SH::YZ_Z / sizeof(E)) + ry * SH::ZROW + zs;
+                os = 1;
+            }
+            int s = pg, ph = 0;
+            for (int n = pg; n < npl; n += NG) {
+                if (!warp_wait_uniform(bar_full + 8 * s, ph, a.token, kNapNs)) return;
+                const int q = q0 + n;
+                if (q >= xa && q <= xe) {
+                    E acc[TY];
+                    if (active) {
+                        const unsigned char* slot = smem + s * SH::SLOT;
+                        pass_item<W, TY>(reinterpret_cast<const E*>(slot) + nb, ns, reinterpret_cast<const S*>(slot) + wb,
+                                         ws, tap4, acc);
+                    }
+                    // the plane slot is free once the outputs are in registers; the result slot is
+                    // reused only after the march has taken its previous plane (7 planes behind)
+                    __syncwarp();
+                    if ((t & 31) == 0) mbar_arrive(bar_empty + 8 * s);
+                    const int m = q - xa;
+                    const int ys = m % SH::RYW;
+                    const unsigned uy = m / SH::RYW;
+                    if (uy >= 1 && !warp_wait_uniform(bar_yempty + 8 * ys, (uy - 1) & 1, a.token, kNapNs)) return;
+                    if (active) {
+                        E* out = reinterpret_cast<E*>(smem + SH::O_YZ + ys * SH::YZ_SLOT) + ob;
+#pragma unroll
+                        for (int o = 0; o < TY; ++o)
+                            if (o >= first) out[o * os] = acc[o];
+                    }
+                    __syncwarp();
+                    if ((t & 31) == 0) mbar_arrive(bar_yfull + 8 * ys);
+                } else {
+                    __syncwarp();
+                    if ((t & 31) == 0) mbar_arrive(bar_empty + 8 * s);
+                }
+                s += NG;
+                if (s >= RW) {
+                    s -= RW;
+                    ph ^= 1;
+                }
+            }
+            return;
         }
-        int s = pg, ph = 0;
-        for (int n = pg; n < npl; n += NG) {
-            if (!warp_wait_uniform(bar_full + 8 * s, ph, a.token, kNapNs)) return;
-            const int q = q0 + n;
-            if (q >= xa && q <= xe) {
+        // Whole warps of one kind: the strides are compile-time offsets of the loads and stores. (In float64
+        // the mixed warps above are the faster ones, 24.7 against 28.2 us per step for one He 65^3 system;
+        // in float32, 64 systems, these are, 519 against 549.)
+        auto planes = [&](auto ns, auto ws, auto os, bool active, int nb, int wb, int ob, int first) {
+            int s = pg, ph = 0, q = q0 + pg;
+            auto next = [&]() {
+                q += NG;
+                s += NG;
+                if (s >= RW) {
+                    s -= RW;
+                    ph ^= 1;
+                }
+            };
+            // a plane before or beyond the chunk has no part in y or z
+            auto pass_by = [&]() -> bool {
+                if (!warp_wait_uniform(bar_full + 8 * s, ph, a.token, kNapNs)) return false;
+                if ((t & 31) == 0) mbar_arrive(bar_empty + 8 * s);
+                next();
+                return true;
+            };
+            while (q < xa)
+                if (!pass_by()) return;
+            for (; q <= xe; next()) {
+                if (!warp_wait_uniform(bar_full + 8 * s, ph, a.token, kNapNs)) return;
                 E acc[TY];
                 if (active) {
                     const unsigned char* slot = smem + s * SH::SLOT;
-                    const E* nodes = reinterpret_cast<const E*>(slot) + nb;
-                    const S* w = reinterpret_cast<const S*>(slot) + wb;
-                    E win[8];
-#pragma unroll
-                    for (int r = 0; r < NROW; ++r) {
-                        win[r & 7] = nodes[r * ns];
-                        if (r >= 7) {
-                            const int rf = r - 7;  // face rf from nodes rf .. rf + 7
-                            // the taps are antisymmetric (tap[7 - j] = -tap[j]): four independent
-                            // differences, then a chain of four (depth 5 instead of 8)
-                            E sum = W::mult(tap(0), W::sub(win[rf & 7], win[(rf + 7) & 7]));
-#pragma unroll
-                            for (int j = 1; j < 4; ++j)
-                                sum = W::fmat(tap(j), W::sub(win[(rf + j) & 7], win[(rf + 7 - j) & 7]), sum);
-                            const E f = W::mult(W::splat(w[rf * ws]), sum);
-                            // face rf reaches outputs o = rf - 7 .. rf with tap o + 7 - rf
-#pragma unroll
-                            for (int o = 0; o < TY; ++o) {
-                                if (o < rf - 7 || o > rf) continue;
-                                acc[o] = (o == rf) ? W::mult_neg(tap(0), f) : W::fmat_k(tap4, o + 7 - rf, f, acc[o]);
-                            }
-                        }
-                    }
+                    pass_item<W, TY>(reinterpret_cast<const E*>(slot) + nb, ns, reinterpret_cast<const S*>(slot) + wb, ws,
+                                     tap4, acc);
                 }
-                // the plane slot is free once the outputs are in registers; the result slot is
-                // reused only after the march has taken its previous plane (7 planes behind)
                 __syncwarp();
                 if ((t & 31) == 0) mbar_arrive(bar_empty + 8 * s);
                 const int m = q - xa;
@@ -1022,15 +1092,23 @@ __global__ void __maxnreg__((wide_max_registers<WideShape<TYW, TZ, sizeof(typena
                 }
                 __syncwarp();
                 if ((t & 31) == 0) mbar_arrive(bar_yfull + 8 * ys);
-            } else {
-                __syncwarp();
-                if ((t & 31) == 0) mbar_arrive(bar_empty + 8 * s);
             }
-            s += NG;
-            if (s >= RW) {
-                s -= RW;
-                ph ^= 1;
-            }
+            while (q < q0 + npl)
+                if (!pass_by()) return;
+        };
+        using One = std::integral_constant<int, 1>;
+        const int wi = (warp - SH::MW) % SH::PWG, lane_id = t & 31;
+        if (wi < SH::YU) {
+            const int zc = wi * 32 + lane_id;
+            planes(std::integral_constant<int, BW>{}, std::integral_constant<int, TZ>{},
+                   std::integral_constant<int, TZ>{}, zc < TZ && z0 + zc < nz, zc + 8, SH::O_W1 / sizeof(S) + zc, zc, 0);
+        } else {
+            const int zi = (wi - SH::YU) * 32 + lane_id;
+            const int ry = zi % TY, seg = zi / TY;
+            const int zs = min(seg * TY, TZ - TY);
+            planes(One{}, One{}, One{}, seg < SH::NZS && y0 + ry < ny && z0 + zs < nz, (ry + HALO) * BW + zs + 1,
+                   SH::O_W2 / sizeof(S) + ry * (TZ + 8) + zs, int(SH::YZ_Z / sizeof(E)) + ry * SH::ZROW + zs,
+                   seg * TY - zs);
         }
         return;
     }
@@ -1073,18 +1151,40 @@ __global__ void __maxnreg__((wide_max_registers<WideShape<TYW, TZ, sizeof(typena
     const int own_off = y * nzp + z;  // this thread's point within a plane of the lane buffer
     int s = 0, sph = 0;   // plane slot and its phase parity
     int ys = 0, yph = 0;  // result slot of the next output completed, and its phase parity
-    for (int n0 = 0; n0 < npl; n0 += 8) {
+    auto release = [&]() {
+        __syncwarp();
+        if ((t & 31) == 0) mbar_arrive(bar_empty + 8 * s);
+        if (++s == RW) {
+            s = 0;
+            sph ^= 1;
+        }
+    };
+    // The 7 planes before a chunk (none before the first) came without their halo and only supply nodes to
+    // the first outputs' x faces. The float64 kernels in 8-row tiles take them in a loop of their own (81 x
+    // 81 x 91, one system: 59 us per step, 61 with a test in the loop), the others skip their work in the
+    // common loop (float64, 13 x 24, one He 65^3 system: 24.7 us per step, 26.7 with a loop of their own).
+    constexpr bool OWN_LOOP = ORB == 2 && TYW == 8;
+    const int first = OWN_LOOP ? xa : q0;
+    if (OWN_LOOP && q0 < xa) {
+#pragma unroll
+        for (int g = 1; g < 8; ++g) {
+            if (!warp_wait_uniform(bar_full + 8 * s, sph, a.token)) return;
+            phq[g] = reinterpret_cast<const E*>(smem + s * SH::SLOT + SH::O_PHI)[own];
+            release();
+        }
+    }
+    const int planes = xe + HALO + 1 - first;
+    for (int n0 = 0; n0 < planes; n0 += 8) {
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
             const int n = n0 + g;
-            if (n >= npl) break;
+            if (n >= planes) break;
             if (!warp_wait_uniform(bar_full + 8 * s, sph, a.token)) return;
             const unsigned char* slot = smem + s * SH::SLOT;
-            const int q = q0 + n;
-            // a plane beyond the chunk came without its halo; one before it (nodes of the first outputs'
-            // x faces) forms nothing
-            phq[g] = reinterpret_cast<const E*>(slot + SH::O_PHI)[q <= xe && q >= xa ? (ty + HALO) * BW + tz + 8 : own];
-            if (q >= xa) {
+            const int q = first + n;
+            // (a plane beyond the chunk came without its halo too)
+            phq[g] = reinterpret_cast<const E*>(slot + SH::O_PHI)[q <= xe && (OWN_LOOP || q >= xa) ? (ty + HALO) * BW + tz + 8 : own];
+            if (OWN_LOOP || q >= xa) {
                 E face;
                 {
                     // antisymmetric taps: sum_j<4 tap[j] (node q-7+j - node q-j)
@@ -1158,12 +1258,7 @@ __global__ void __maxnreg__((wide_max_registers<WideShape<TYW, TZ, sizeof(typena
                 // on the previous plane); its y+z part joins when it completes
                 acc[g] = W::mult_neg(tap(0), face);
             }
-            __syncwarp();
-            if ((t & 31) == 0) mbar_arrive(bar_empty + 8 * s);
-            if (++s == RW) {
-                s = 0;
-                sph ^= 1;
-            }
+            release();
         }
     }
 }
@@ -1755,7 +1850,7 @@ Tile choose_tile(int ny, int nzp) {
 // launch decide the CTA count, the waves, the padding and the halo work; which wins depends on the
 // grid, the lane count and the GPU. With the autotuner
 // on, the first filter call for a (device, grid, precision, lanes) key times every candidate on the
-// call's own buffers (the first Chebyshev step, which the real run then recomputes), keeps the
+// call's own buffers (a Chebyshev step, whose output the real run then overwrites), keeps the
 // fastest in a host table, and every later filter or apply launch for that key uses it. Every
 // candidate gives bit-identical results: each output is formed by the same arithmetic in the same
 // order whatever the tiling. Off, the heuristics choose_tile / choose_chunk decide.
@@ -1785,10 +1880,11 @@ bool tuned_choice(const TuneKey& key, TileChoice* out) {
     return true;
 }
 
-// Times every candidate tiling (the geometry's padded rows are in place): one untimed launch, then three timed ones each. With apply null,
-// the launch is the first Chebyshev step (packed block in buf[2] -> buf[0]); otherwise it is the
-// apply described by *apply (packed block in buf[2], written to the caller's output, which the
-// real launch then rewrites). Synchronises the stream.
+// Times every candidate tiling (the geometry's padded rows are in place): one untimed launch, then the
+// best of three times three each. With apply null, the launch is a Chebyshev step (packed block in buf[2],
+// previous iterate in buf[1] -> buf[0]); otherwise it is the apply described by *apply (packed block in
+// buf[2], written to the caller's output, which the real launch then rewrites). Synchronises the stream.
+constexpr int kTunedChunks = 7;  // x chunks tried (a chunk's halo planes are cheap, so short ones can win)
 template <typename Lane>
 int tune_slab(const cdftb_operator* op, int64_t batch, void* geo_base, void* buf[3], int64_t lanes,
               const double* coefficients, int degree, cudaStream_t stream, TileChoice* best,
@@ -1816,30 +1912,37 @@ int tune_slab(const cdftb_operator* op, int64_t batch, void* geo_base, void* buf
         if (apply) {
             a = *apply;
         } else {
+            // a step with a previous iterate, as all but the first are (what buf[1] holds does not matter)
             a.coef = coefficients;
             a.degree = degree;
             a.step = 0;
-            a.has_prev = 0;
+            a.has_prev = degree > 1;
             a.final_out = 0;
             a.out = buf[0];
             a.out_dtype = 0;
+            CUtensorMap unused;
+            if ((st = encode_lanes<Lane>(buf[1], nzp, ny, nx, lanes, ty, tz, &unused, &m.prev)) != CDFTB_OK) break;
         }
         const int64_t tiles = int64_t(ceil_div(ny, ty)) * ceil_div(nzp, tz);
-        int chunks_list[5] = {1, 2, 3, 4, 0};
-        chunks_list[4] = static_cast<int>(ceil_div(nx, choose_chunk(nx, tiles * lanes, sm_count())));
-        for (int c = 0; c < 5 && st == CDFTB_OK; ++c) {
-            const int chunks = chunks_list[c];
-            if (chunks < 1 || (c == 4 && chunks <= 4)) continue;  // the heuristic's chunk, when not already tried
+        const int heuristic = static_cast<int>(ceil_div(nx, choose_chunk(nx, tiles * lanes, sm_count())));
+        for (int c = 1; c <= kTunedChunks + 1 && st == CDFTB_OK; ++c) {
+            const int chunks = c <= kTunedChunks ? c : heuristic;
+            if (c > kTunedChunks && chunks <= kTunedChunks) continue;  // the heuristic's chunk, when not already tried
             const int xchunk = static_cast<int>(ceil_div(nx, chunks));
             if (chunks > 1 && (xchunk < 8 || ceil_div(nx, xchunk) != chunks)) continue;
+            float ms = -1.0f;
             if ((st = launch_tz<Lane>(ty, tz, m, a, lanes, stream, xchunk)) != CDFTB_OK) break;
-            if ((st = check(cudaEventRecord(e0, stream))) != CDFTB_OK) break;
-            for (int r = 0; r < 3 && st == CDFTB_OK; ++r) st = launch_tz<Lane>(ty, tz, m, a, lanes, stream, xchunk);
+            for (int round = 0; round < 3 && st == CDFTB_OK; ++round) {
+                if ((st = check(cudaEventRecord(e0, stream))) != CDFTB_OK) break;
+                for (int r = 0; r < 3 && st == CDFTB_OK; ++r) st = launch_tz<Lane>(ty, tz, m, a, lanes, stream, xchunk);
+                if (st != CDFTB_OK) break;
+                if ((st = check(cudaEventRecord(e1, stream))) != CDFTB_OK) break;
+                if ((st = check(cudaEventSynchronize(e1))) != CDFTB_OK) break;
+                float t = 0.0f;
+                if ((st = check(cudaEventElapsedTime(&t, e0, e1))) != CDFTB_OK) break;
+                if (ms < 0.0f || t < ms) ms = t;
+            }
             if (st != CDFTB_OK) break;
-            if ((st = check(cudaEventRecord(e1, stream))) != CDFTB_OK) break;
-            if ((st = check(cudaEventSynchronize(e1))) != CDFTB_OK) break;
-            float ms = 0.0f;
-            if ((st = check(cudaEventElapsedTime(&ms, e0, e1))) != CDFTB_OK) break;
             if (best_ms < 0.0f || ms < best_ms) {
                 best_ms = ms;
                 *best = TileChoice{ty, tz, xchunk};
