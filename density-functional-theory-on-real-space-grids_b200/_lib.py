@@ -42,6 +42,8 @@ SIGNATURES: dict[str, tuple] = {
     "cdftb_launch_count": (ctypes.c_ulonglong, []),
     "cdftb_weighted_divergence_f64": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p,
                                               c_void_p, c_double, c_int, c_void_p]),
+    "cdftb_cusp_apply_adjoint_f64": (c_int, [ctypes.POINTER(Operator), c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
+                                             c_void_p, c_int64, c_void_p]),
     "cdftb_cusp_apply_work_bytes": (c_int64, [ctypes.POINTER(Operator), c_int64]),
     "cdftb_cusp_apply": (c_int, [ctypes.POINTER(Operator), c_void_p, c_int, c_void_p, c_int, c_int64, c_int, c_void_p,
                                  c_int64, c_void_p]),

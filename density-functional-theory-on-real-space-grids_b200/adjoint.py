@@ -30,9 +30,13 @@ total energies on a fixed, unanchored grid) is the check.
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 
+from . import _lib
+from ._lib import call, ptr, stream_handle
 from .operators import weighted_divergence
 from .xc import functional_by_name
 
@@ -54,12 +58,33 @@ class CuspApply(torch.autograd.Function):
         grid = h.grid
         n = grid.n_points
         y = y_bar.contiguous()
+        # Order 8 in float64 with one potential: three launches of the slab apply's kind. The sum over orbitals
+        # below can itself be differentiated, so a backward pass that records a graph goes through torch, as do
+        # the other orders and mixed types.
+        if (grid.fd_order == 8 and h.dtype == torch.float64 and not torch.is_grad_enabled() and y.numel()
+                and potential.shape == (n,) and phi.shape == y.shape
+                and all(t.dtype == torch.float64 and t.device == h._inv.device for t in (y, phi, potential))):
+            return _native_vjp(ctx, h, y, phi.contiguous(), potential.contiguous())
         scaled = (h._inverse_weight * y).reshape(-1, *grid.shape)
         div = weighted_divergence(scaled, h.factor.face_weights(grid.fd_order), grid.spacing, grid.fd_order,
                                   grid.shape).reshape(y.shape)
         phi_bar = 0.5 * div + potential * y
         potential_bar = (y * phi).reshape(-1, n).sum(dim=0)
         return phi_bar, potential_bar, None
+
+
+def _native_vjp(ctx, hamiltonian, y, phi, potential):
+    """``(phi_bar, potential_bar, None)`` of the order-8 float64 apply by ``cdftb_cusp_apply_adjoint_f64``."""
+    n = hamiltonian.grid.n_points
+    batch = y.numel() // n
+    op = hamiltonian.operator(potential)
+    phi_bar = torch.empty_like(y)
+    potential_bar = torch.empty_like(potential) if ctx.needs_input_grad[1] else None
+    nbytes = _lib.library().cdftb_cusp_apply_work_bytes(ctypes.byref(op), batch)
+    work = torch.empty(nbytes, dtype=torch.uint8, device=y.device)
+    call("cdftb_cusp_apply_adjoint_f64", ctypes.byref(op), ptr(y), ptr(phi), ptr(phi_bar), ptr(potential_bar), batch,
+         ptr(work), nbytes, stream_handle(y.device))
+    return phi_bar, potential_bar, None
 
 
 class PoissonSolve(torch.autograd.Function):

@@ -1326,13 +1326,14 @@ constexpr int kPrepThreads = 256;
 constexpr int kPrepPerBlock = 4 * kPrepThreads;
 
 struct PadJob {
-    const void* src;         // null: zeros
+    const void* src;         // null: fill
     void* dst;
     int64_t total;           // elements written
     int cols, cols_pad;      // source row -> padded row (zeros behind)
     int64_t group_rows;      // rows per group and the groups' distance in the source
     int64_t group_stride;
     int64_t first_block;
+    double fill;             // the value of a row's own columns without a source
 };
 
 struct PrepArgs {
@@ -1341,13 +1342,14 @@ struct PrepArgs {
     int64_t lane_blocks;     // CTAs per lane
     const void* block;
     int block_dtype;
+    const void* scale;       // a factor per point for the block (wide lanes), or null
     int64_t batch;
     int nx, ny, nz, nzp;
     int opg, lpg;
     void* lanes;
 };
 
-template <typename L>
+template <typename L, bool SCALED>
 __global__ void __launch_bounds__(kPrepThreads) prep_kernel(const __grid_constant__ PrepArgs a) {
     using S = typename L::S;
     const int64_t b = blockIdx.x;
@@ -1364,10 +1366,14 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(const __grid_constan
         for (int u = 0; u < kPrepPerBlock / kPrepThreads; ++u) {
             const int64_t k = base + u * kPrepThreads;
             v[u] = S(0);
-            if (k >= job.total || !src) continue;
+            if (k >= job.total) continue;
             const int64_t row = narrow ? static_cast<unsigned>(k) / static_cast<unsigned>(job.cols_pad) : k / job.cols_pad;
             const int c = static_cast<int>(k - row * job.cols_pad);
             if (c >= job.cols) continue;
+            if (!src) {
+                v[u] = static_cast<S>(job.fill);
+                continue;
+            }
             const int64_t g = job.group_rows > row ? 0 : row / job.group_rows;
             v[u] = src[g * job.group_stride + (row - g * job.group_rows) * job.cols + c];
         }
@@ -1398,6 +1404,11 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(const __grid_constan
 #pragma unroll
             for (int h = 0; h < ORB; ++h)
                 v[u][h] = in && orb[h] >= 0 ? load_as<S>(a.block, a.block_dtype, orb[h] * n_points + pt) : S(0);
+            if constexpr (SCALED) {
+                const S f = in ? static_cast<const S*>(a.scale)[pt] : S(0);
+#pragma unroll
+                for (int h = 0; h < ORB; ++h) v[u][h] *= f;
+            }
         }
 #pragma unroll
         for (int u = 0; u < kPrepPerBlock / kPrepThreads; ++u)
@@ -1574,9 +1585,11 @@ struct GeoCopies {
 };
 
 // The jobs that copy the geometry into the padded rows TMA reads; without_potential zeroes the
-// potential rows instead of copying them. Returns the CTAs they take.
+// potential rows instead of copying them, and an operator without h^3/omega gets inv_fill there. Returns
+// the CTAs they take.
 template <typename Lane>
-int64_t geometry_jobs(const cdftb_operator* op, int64_t batch, void* geo_base, bool without_potential, PrepArgs* args) {
+int64_t geometry_jobs(const cdftb_operator* op, int64_t batch, void* geo_base, bool without_potential, double inv_fill,
+                      PrepArgs* args) {
     using S = typename Lane::S;
     const int64_t nx = op->nx, ny = op->ny, nz = op->nz;
     const GeoPack gp = geo_pack(op, batch);
@@ -1586,7 +1599,8 @@ int64_t geometry_jobs(const cdftb_operator* op, int64_t batch, void* geo_base, b
     int64_t blocks = 0;
     auto job = [&](int i, const void* src, void* dst, int64_t rows, int64_t cols, int cols_pad, int64_t group_rows,
                    int64_t group_stride) {
-        args->pad[i] = PadJob{src, dst, rows * cols_pad, static_cast<int>(cols), cols_pad, group_rows, group_stride, blocks};
+        args->pad[i] = PadJob{src,        dst,          rows * cols_pad, static_cast<int>(cols), cols_pad,
+                              group_rows, group_stride, blocks,          i == 3 ? inv_fill : 0.0};
         blocks += ceil_div(rows * cols_pad, kPrepPerBlock);
     };
     auto whole = [&](int i, const void* src, void* dst, int64_t rows, int64_t cols, int cols_pad) {
@@ -1780,16 +1794,18 @@ int encode_lanes(void* buf, int nzp, int ny, int nx, int64_t lanes, int ty, int 
 // The call's copies: the caller's block into lanes at dst, the geometry into padded rows at geo_base.
 template <typename L>
 int prepare(const cdftb_operator* op, const void* block, int in_dtype, int64_t batch, int64_t lanes, void* dst,
-            void* geo_base, bool without_potential, cudaStream_t stream) {
+            void* geo_base, bool without_potential, cudaStream_t stream, const void* scale = nullptr,
+            double inv_fill = 0.0) {
     if ((reinterpret_cast<uintptr_t>(dst) & 15) != 0) return CDFTB_ERR_ARGUMENT;
     PrepArgs a{};
-    int64_t blocks = geometry_jobs<L>(op, batch, geo_base, without_potential || !op->potential, &a);
+    int64_t blocks = geometry_jobs<L>(op, batch, geo_base, without_potential || !op->potential, inv_fill, &a);
     a.pack_first = blocks;
     const int nzp = padded_z(op->nz);
     if constexpr (L::WIDE) {
         a.lane_blocks = ceil_div(int64_t(op->nx) * op->ny * nzp, kPrepPerBlock);
         a.block = block;
         a.block_dtype = in_dtype;
+        a.scale = scale;
         a.batch = batch;
         a.nx = op->nx;
         a.ny = op->ny;
@@ -1800,11 +1816,19 @@ int prepare(const cdftb_operator* op, const void* block, int in_dtype, int64_t b
         a.lanes = dst;
         blocks += lanes * a.lane_blocks;
     } else {
+        if (scale) return CDFTB_ERR_ARGUMENT;  // 8-byte lanes are packed without a factor
         const int st = pack_block<L>(op, block, in_dtype, batch, op->nx, op->ny, op->nz, nzp, lanes, dst, stream);
         if (st != CDFTB_OK) return st;
     }
     if (blocks > 0x7fffffffll) return CDFTB_ERR_CAPACITY;
-    prep_kernel<L><<<static_cast<unsigned>(blocks), kPrepThreads, 0, stream>>>(a);
+    if constexpr (L::WIDE) {
+        if (scale)
+            prep_kernel<L, true><<<static_cast<unsigned>(blocks), kPrepThreads, 0, stream>>>(a);
+        else
+            prep_kernel<L, false><<<static_cast<unsigned>(blocks), kPrepThreads, 0, stream>>>(a);
+    } else {
+        prep_kernel<L, false><<<static_cast<unsigned>(blocks), kPrepThreads, 0, stream>>>(a);
+    }
     return check_launch();
 }
 
@@ -2014,7 +2038,7 @@ int slab_filter(const cdftb_operator* op, const void* block, int in_dtype, void*
 
 template <typename Lane>
 int slab_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* out, int out_dtype, void* work,
-               int64_t batch, int kinetic_only, cudaStream_t stream) {
+               int64_t batch, int kinetic_only, cudaStream_t stream, const void* scale = nullptr, double inv_fill = 0.0) {
     const int nx = op->nx, ny = op->ny, nz = op->nz;
     const int nzp = padded_z(nz);
     const int64_t lanes = lane_count<Lane>(op, batch);
@@ -2024,7 +2048,8 @@ int slab_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* ou
     TileChoice choice{t0.ty, t0.tz, 0};
     const TuneKey key = tune_key(op, lanes, Lane::WIDE);
     const bool known = tuned_choice(key, &choice);
-    int st = prepare<Lane>(op, phi, in_dtype, batch, lanes, w, w + lanes * lane_bytes, kinetic_only != 0, stream);
+    int st = prepare<Lane>(op, phi, in_dtype, batch, lanes, w, w + lanes * lane_bytes, kinetic_only != 0, stream,
+                           scale, inv_fill);
     if (st != CDFTB_OK) return st;
     bool autotune;
     {
@@ -2059,6 +2084,29 @@ int slab_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* ou
     a.out = out;
     a.out_dtype = out_dtype;
     return launch_tz<Lane>(ty, tz, m, a, lanes, stream, choice.xchunk);
+}
+
+// The end of the adjoint apply: out = 0.5 Div(D y) from the slab kernel, phi_bar = out + V y, and
+// potential_bar = sum over the orbitals of y phi, in one pass (three reads and a write per value): 28 us
+// for 5 orbitals at 101^3, what HBM at its copy rate takes for those bytes. The whole backward pass there, with
+// D y formed while the lanes are packed, takes 147 us; the stencil over caller layout (197 us) and torch's
+// four elementwise passes took 320.
+__global__ void __launch_bounds__(256) adjoint_finish_kernel(const double* __restrict__ y,
+                                                             const double* __restrict__ phi,
+                                                             const double* __restrict__ potential, int64_t batch,
+                                                             int64_t n, double* __restrict__ out,
+                                                             double* __restrict__ potential_bar) {
+    const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (p >= n) return;
+    const double v = potential[p];
+    double sum = 0.0;
+#pragma unroll 4
+    for (int64_t b = 0; b < batch; ++b) {
+        const double yb = y[b * n + p];
+        out[b * n + p] = fma(v, yb, out[b * n + p]);
+        if (potential_bar) sum = fma(yb, phi[b * n + p], sum);
+    }
+    if (potential_bar) potential_bar[p] = sum;
 }
 
 // Wide lanes serve every filter and apply with one shared geometry (lanes need not follow orbital
@@ -2228,4 +2276,28 @@ extern "C" int cdftb_cusp_apply(const cdftb_operator* op, const void* phi, int i
     if (op->dtype == CDFTB_F32)
         return cdftb::slab_apply<cdftb::LaneF2>(op, phi, in_dtype, out, out_dtype, work, batch, kinetic_only, s);
     return cdftb::slab_apply<cdftb::LaneD>(op, phi, in_dtype, out, out_dtype, work, batch, kinetic_only, s);
+}
+
+extern "C" int cdftb_cusp_apply_adjoint_f64(const cdftb_operator* op, const double* y, const double* phi, double* phi_bar,
+                                            double* potential_bar, int64_t batch, void* work, int64_t work_bytes,
+                                            cdftb_stream_t stream) {
+    if (!op || !y || !phi_bar || (potential_bar && !phi) || batch < 1) return CDFTB_ERR_ARGUMENT;
+    if (op->dtype != CDFTB_F64 || !cdftb::slab_filter_applies(op) || op->per_system_geometry ||
+        op->potential_stride != 0 || !(op->spacing > 0.0) || !op->face_weights[0] || !op->face_weights[1] ||
+        !op->face_weights[2] || !op->inverse_weight || !op->potential || !work ||
+        reinterpret_cast<uintptr_t>(work) % 16 != 0 ||
+        work_bytes < cdftb::slab_apply_work_bytes(op, batch))
+        return CDFTB_ERR_ARGUMENT;
+    // the kinetic apply forms 0.5 inv div: with h^3/omega in the lanes and inv = 1 that is 0.5 div
+    cdftb_operator div = *op;
+    div.inverse_weight = nullptr;
+    div.potential = nullptr;
+    cudaStream_t s = cdftb::as_stream(stream);
+    int st = cdftb::slab_apply<cdftb::WideD2>(&div, y, CDFTB_F64, phi_bar, CDFTB_F64, work, batch, 1, s,
+                                              op->inverse_weight, 1.0);
+    if (st != CDFTB_OK) return st;
+    const int64_t n = int64_t(op->nx) * op->ny * op->nz;
+    cdftb::adjoint_finish_kernel<<<static_cast<unsigned>(cdftb::ceil_div(n, 256)), 256, 0, s>>>(
+        y, phi, static_cast<const double*>(op->potential), batch, n, phi_bar, potential_bar);
+    return cdftb::check_launch();
 }

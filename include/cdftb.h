@@ -79,6 +79,14 @@ int cdftb_weighted_divergence_f64(const double* box, double* out, int64_t batch,
                                   const double* w0, const double* w1, const double* w2, double spacing,
                                   int accuracy, cdftb_stream_t stream);
 
+/* The vector-Jacobian product of the order-8 float64 apply with one potential (no reference
+ * counterpart: the reference differentiates by autograd): phi_bar = 0.5 Div((h^3/omega) y) + V y, and
+ * potential_bar = sum over the batch of y phi (NULL leaves it out; phi may then be NULL). Scratch:
+ * cdftb_cusp_apply_work_bytes of the operator. */
+int cdftb_cusp_apply_adjoint_f64(const cdftb_operator* op, const double* y, const double* phi, double* phi_bar,
+                                 double* potential_bar, int64_t batch, void* work, int64_t work_bytes,
+                                 cdftb_stream_t stream);
+
 /* (a2) out = A phi for a batch of orbitals (src/cdft/operators/hamiltonian.py:251-318,
  * apply / apply_with_potential / kinetic_apply). out may be double or float (out_dtype).
  * kinetic_only = 1 drops the V phi term (hamiltonian.py:303). With device scratch of at least
@@ -112,7 +120,7 @@ int cdftb_chebyshev_filter(const cdftb_operator* op, const void* block, int in_d
 /* No reference counterpart (the reference has no kernels of its own to tune): the tile autotuner of
  * the order-8 slab kernels. With it enabled, the first cdftb_chebyshev_filter or cdftb_cusp_apply
  * call for a (device, grid, precision, lane count) key times each candidate tiling -- z tiles of 32
- * or 36 columns, 1 to 4 x chunks and the heuristic's chunk -- on that call's own buffers, keeps the
+ * or 36 columns, 1 to 7 x chunks and the heuristic's chunk -- on that call's own buffers, keeps the
  * fastest, and every later filter or apply launch for the key uses it. That first call synchronises
  * its stream (make it before any stream capture); results are bit-identical whatever the tiling. Disabled (the
  * default in the C library), heuristics choose the tiling. cdftb_filter_tuned_tile reports the
