@@ -142,6 +142,36 @@ __device__ __forceinline__ double far_factor(const Nuclei& nuc, const double* p)
     return far;
 }
 
+// The nodes of the spheres, a CTA per shell: node = centre + r (sin cos, sin sin, cos), weight =
+// wr w_cos. Every product and sum rounds by itself (no FMA), as the formula over arrays does: a node on a
+// grid plane stays there. A few us for ~2 x 10^5 nodes; a shell's tables (7 n doubles) stay in L1.
+__global__ void __launch_bounds__(256) sphere_nodes_kernel(int n_shells, int n_spheres, const int4* __restrict__ shells,
+                                                           const double* __restrict__ tables, int64_t m,
+                                                           double* __restrict__ points, double* __restrict__ base,
+                                                           int* __restrict__ owner) {
+    const int4 s = shells[blockIdx.x];  // first node, polar order, place of its tables, sphere
+    const double r = tables[blockIdx.x];
+    const double wr = tables[n_shells + blockIdx.x];
+    const double* centre = tables + 2 * n_shells + 3 * s.w;
+    const double cx = centre[0], cy = centre[1], cz = centre[2];
+    const int n = s.y, n_phi = 2 * n;
+    const double* cos_phi = tables + 2 * n_shells + 3 * n_spheres + s.z;
+    const double* sin_phi = cos_phi + n_phi;
+    const double* sin_theta = sin_phi + n_phi;
+    const double* cos_theta = sin_theta + n;
+    const double* weight = cos_theta + n;
+    for (int k = threadIdx.x; k < n * n_phi; k += blockDim.x) {
+        const int i = k / n_phi, j = k - i * n_phi;
+        const int64_t node = int64_t(s.x) + k;
+        if (node >= m) return;
+        points[3 * node] = __dadd_rn(__dmul_rn(r, __dmul_rn(sin_theta[i], cos_phi[j])), cx);
+        points[3 * node + 1] = __dadd_rn(__dmul_rn(r, __dmul_rn(sin_theta[i], sin_phi[j])), cy);
+        points[3 * node + 2] = __dadd_rn(__dmul_rn(r, cos_theta[i]), cz);
+        base[node] = __dmul_rn(wr, weight[i]);
+        owner[node] = s.w;
+    }
+}
+
 // Node fields: partition P (quadrature.py:393-419), weights = base * P, u, grad u, f^2, W.
 __global__ void node_fields_kernel(Nuclei nuc, const double* __restrict__ pts, const int* __restrict__ owner,
                                    const double* __restrict__ base_w, int64_t m, double* __restrict__ partition,
@@ -410,6 +440,16 @@ extern "C" int cdftb_geometry_face_weights(int n_atoms, const double* charges, c
         if (st != CDFTB_OK) return st;
     }
     return CDFTB_OK;
+}
+
+extern "C" int cdftb_geometry_sphere_nodes(int n_shells, int n_spheres, const int* shells, const double* tables, int64_t m,
+                                           double* points, double* base, int* owner, cdftb_stream_t stream) {
+    if (n_shells < 1 || n_spheres < 1 || n_spheres > MAX_ATOMS || m < 1 || m > 0x7fffffffll || !shells || !tables ||
+        !points || !base || !owner || reinterpret_cast<uintptr_t>(shells) % 16 != 0)
+        return CDFTB_ERR_ARGUMENT;
+    sphere_nodes_kernel<<<static_cast<unsigned>(n_shells), 256, 0, as_stream(stream)>>>(
+        n_shells, n_spheres, reinterpret_cast<const int4*>(shells), tables, m, points, base, owner);
+    return check_launch();
 }
 
 extern "C" int cdftb_geometry_node_fields(int n_atoms, const double* charges, const double* positions,

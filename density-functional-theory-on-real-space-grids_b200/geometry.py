@@ -150,27 +150,53 @@ class CuspFactor:
         return out
 
 
-def sphere_rule(centre: np.ndarray, radius_sphere: float, spacing: float, radial_order: int, node_spacing: float):
-    """Node positions and bare weights ``r^2 dr dOmega`` of one sphere (``quadrature.py:123-182``)."""
+def sphere_shells(radius_sphere: float, spacing: float, radial_order: int, node_spacing: float):
+    """The shells of one sphere (``quadrature.py:123-182``): radii, weights ``r^2 dr``, polar orders."""
     n_panels = max(2, int(math.ceil(radius_sphere / spacing)))
     edges = np.linspace(0.0, radius_sphere, n_panels + 1)
     gl_nodes, gl_weights = gauss_legendre(radial_order)
-    points, weights = [], []
-    for lo, hi in zip(edges[:-1], edges[1:]):
-        mid, half = 0.5 * (hi + lo), 0.5 * (hi - lo)
-        for node, weight in zip(gl_nodes, gl_weights):
-            r = mid + half * node
-            wr = half * weight * r * r
-            n_theta = max(4, int(math.ceil(math.sqrt(2.0 * math.pi) * r / (node_spacing * spacing))))
-            n_phi = 2 * n_theta
-            cos_nodes, cos_weights = gauss_legendre(n_theta)
-            phis = 2.0 * math.pi * (np.arange(n_phi) + 0.5) / n_phi
-            sin_theta = np.sqrt(np.clip(1.0 - cos_nodes ** 2, 0.0, 1.0))
-            directions = np.stack([np.outer(sin_theta, np.cos(phis)).ravel(), np.outer(sin_theta, np.sin(phis)).ravel(),
-                                   np.repeat(cos_nodes, n_phi)], axis=1)
-            points.append(r * directions)
-            weights.append(wr * (np.repeat(cos_weights, n_phi) * (2.0 * math.pi / n_phi)))
-    return np.concatenate(points) + centre, np.concatenate(weights)
+    mid, half = 0.5 * (edges[1:] + edges[:-1]), 0.5 * (edges[1:] - edges[:-1])
+    r = mid[:, None] + half[:, None] * gl_nodes
+    wr = half[:, None] * gl_weights * r * r
+    orders = np.maximum(4, np.ceil(math.sqrt(2.0 * math.pi) * r / (node_spacing * spacing)).astype(np.int64))
+    return r.reshape(-1), wr.reshape(-1), orders.reshape(-1)
+
+
+def sphere_nodes(centres, shells, device):
+    """Node positions ``(M, 3)``, bare weights ``r^2 dr dOmega`` and owners of the spheres, on the device.
+
+    A shell of polar order n carries the product rule of n Gauss--Legendre and 2n uniform angles
+    (``quadrature.py:123-182``); the host forms the tables per order, the kernel the products, in the order
+    (and so with the bits) of the formula over whole arrays. Forming the ~2 x 10^5 nodes of two spheres
+    here shell by shell and copying them took 5 ms.
+    """
+    radii = np.concatenate([s[0] for s in shells])
+    weights = np.concatenate([s[1] for s in shells])
+    orders = np.concatenate([s[2] for s in shells])
+    atoms = np.repeat(np.arange(len(shells)), [s[0].size for s in shells])
+    tables, place, at = [], {}, 0
+    for order in np.unique(orders):
+        n = int(order)
+        cos_nodes, cos_weights = gauss_legendre(n)
+        phis = 2.0 * math.pi * (np.arange(2 * n) + 0.5) / (2 * n)
+        sin_theta = np.sqrt(np.clip(1.0 - cos_nodes ** 2, 0.0, 1.0))
+        tables += [np.cos(phis), np.sin(phis), sin_theta, cos_nodes, cos_weights * (2.0 * math.pi / (2 * n))]
+        place[n] = at
+        at += 7 * n
+    counts = 2 * orders * orders
+    first = np.cumsum(counts) - counts
+    m = int(counts.sum())
+    if m > np.iinfo(np.int32).max:
+        raise ValueError(f"{m} quadrature nodes; at most 2^31 - 1 are supported")
+    ints = np.stack([first, orders, np.array([place[int(n)] for n in orders]), atoms], axis=1).astype(np.int32)
+    reals = np.concatenate([radii, weights, np.asarray(centres, dtype=np.float64).reshape(-1), *tables])
+    ints_d, reals_d = torch.from_numpy(np.ascontiguousarray(ints)).to(device), torch.from_numpy(reals).to(device)
+    points = torch.empty((m, 3), dtype=torch.float64, device=device)
+    base = torch.empty(m, dtype=torch.float64, device=device)
+    owner = torch.empty(m, dtype=torch.int32, device=device)
+    call("cdftb_geometry_sphere_nodes", radii.size, len(shells), ptr(ints_d), ptr(reals_d), m, ptr(points), ptr(base),
+         ptr(owner), stream_handle(device))
+    return points, base, owner
 
 
 def _interp_matrix(n: int, refine: int, origin: float, h: float, degree: int = 7):
@@ -184,20 +210,23 @@ def _interp_matrix(n: int, refine: int, origin: float, h: float, degree: int = 7
     t = fractional - first.astype(np.float64)
     x = t[:, None] - np.arange(k, dtype=np.float64)[None, :]
     w = np.ones_like(x)
-    for j in range(k):
-        for m in range(k):
-            if m != j:
-                w[:, j] = w[:, j] * x[:, m] / float(j - m)
+    for m in range(k):  # every column j times x_m / (j - m), the column m as it is
+        factor = np.repeat(x[:, m:m + 1], k, axis=1)
+        factor[:, m] = 1.0
+        distance = np.arange(k, dtype=np.float64) - m
+        distance[m] = 1.0
+        w = w * factor / distance
     matrix = np.zeros((n, n_fine))
     rows = (first[:, None] + np.arange(k)[None, :]).reshape(-1)
     cols = np.repeat(np.arange(n_fine), k)
-    np.add.at(matrix, (rows, cols), w.reshape(-1))
-    lo = np.zeros(n, dtype=np.int32)
-    hi = np.zeros(n, dtype=np.int32)
-    for c in range(n):
-        nz = np.nonzero((first <= c) & (c < first + k))[0]
-        lo[c], hi[c] = (nz.min(), nz.max() + 1) if nz.size else (0, 0)
-    return fine, matrix, lo, hi
+    matrix[rows, cols] = w.reshape(-1)
+    # first does not fall: the fine points with first <= c < first + k are neighbours
+    c = np.arange(n)
+    lo = np.searchsorted(first, c - k, side="right")
+    hi = np.searchsorted(first, c, side="right")
+    none = hi <= lo
+    lo[none] = hi[none] = 0
+    return fine, matrix, lo.astype(np.int32), hi.astype(np.int32)
 
 
 class CuspQuadrature:
@@ -227,7 +256,7 @@ class CuspQuadrature:
         origin = np.asarray(grid.origin)
         upper = origin + np.array([(n - 1) * h for n in grid.shape])
         margin = (self.degree // 2 + 1.5) * h
-        self.taper, self.overlapping, spheres, pts, owner, base = [], [], [], [], [], []
+        self.taper, self.overlapping, spheres, shells = [], [], [], []
         for atom in range(n_atoms):
             centre = positions[atom]
             edge_distance = float(np.minimum(centre - origin, upper - centre).min())
@@ -247,19 +276,13 @@ class CuspQuadrature:
                 others = np.concatenate([positions[:atom], positions[atom + 1:]])
                 overlapping = float(np.sqrt(((others - centre) ** 2).sum(axis=-1)).min()) < 2.0 * radius
             self.overlapping.append(overlapping)
-            p, w = sphere_rule(centre, radius, h, self.radial_order,
-                               self.node_spacing_overlapping if overlapping else self.node_spacing)
+            shells.append(sphere_shells(radius, h, self.radial_order,
+                                        self.node_spacing_overlapping if overlapping else self.node_spacing))
             spheres.append([*centre, radius, taper_centre, width])
-            pts.append(p)
-            base.append(w)
-            owner.append(np.full(p.shape[0], atom, dtype=np.int32))
         self.sphere_rows = _host(spheres)
-        self.n_nodes = int(sum(p.shape[0] for p in pts))
-        m = self.n_nodes
         f = dict(dtype=torch.float64, device=dev)
-        self.points = torch.from_numpy(np.ascontiguousarray(np.concatenate(pts))).to(dev)
-        owner_d = torch.from_numpy(np.concatenate(owner)).to(dev)
-        base_d = torch.from_numpy(np.ascontiguousarray(np.concatenate(base))).to(dev)
+        self.points, base_d, owner_d = sphere_nodes(positions, shells, dev)
+        m = self.n_nodes = self.points.shape[0]
         self.partition = torch.empty(m, **f)
         self.weights = torch.empty(m, **f)
         self.f2 = torch.empty(m, **f)
@@ -335,10 +358,13 @@ class CuspQuadrature:
         h = grid.spacing
         refine = self.far_refine
         axes = [_interp_matrix(n, refine, o, h, self.degree) for n, o in zip(grid.shape, grid.origin)]
-        t = [torch.from_numpy(np.ascontiguousarray(a[0])).to(dev) for a in axes]
-        mats = [torch.from_numpy(np.ascontiguousarray(a[1])).to(dev) for a in axes]
-        los = [torch.from_numpy(a[2]).to(dev) for a in axes]
-        his = [torch.from_numpy(a[3]).to(dev) for a in axes]
+        reals = torch.from_numpy(np.concatenate([x.reshape(-1) for a in axes for x in a[:2]])).to(dev)
+        bands = torch.from_numpy(np.concatenate([x for a in axes for x in a[2:]])).to(dev)
+        sizes = [x.size for a in axes for x in a[:2]]
+        (t0, m0, t1, m1, t2, m2) = reals.split(sizes)
+        t, mats = [t0, t1, t2], [m0, m1, m2]
+        (l0, h0, l1, h1, l2, h2) = bands.split([x.size for a in axes for x in a[2:]])
+        los, his = [l0, l1, l2], [h0, h1, h2]
         nx, ny, nz = grid.shape
         work = torch.empty(nx * refine * ny * refine * nz + nx * ny * refine * nz, dtype=torch.float64, device=dev)
         out = torch.empty(grid.n_points, dtype=torch.float64, device=dev)

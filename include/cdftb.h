@@ -458,6 +458,13 @@ int cdftb_geometry_cusp_fields(int n_atoms, const double* charges, const double*
 int cdftb_geometry_face_weights(int n_atoms, const double* charges, const double* positions, int nx, int ny, int nz,
                                 double ox, double oy, double oz, double spacing, int accuracy, double* w0, double* w1,
                                 double* w2, int* underflow, cdftb_stream_t stream);
+/* The nodes of the quadrature spheres (quadrature.py:123-182): positions (m, 3), bare weights and owning
+ * sphere. shells (n_shells, 4): first node, polar order n (2 n^2 nodes), place of the order's tables,
+ * sphere. tables: the shells' radii, their weights r^2 dr, the spheres' centres (n_spheres, 3), then per
+ * order cos phi (2n), sin phi (2n), sin theta (n), cos theta (n), weights w_cos 2 pi / 2n (n). Device
+ * arrays; m is the sum of the shells' nodes. */
+int cdftb_geometry_sphere_nodes(int n_shells, int n_spheres, const int* shells, const double* tables, int64_t m,
+                                double* points, double* base, int* owner, cdftb_stream_t stream);
 /* Node partition P, weights = base P, f^2, grad u and W at the sphere nodes (quadrature.py:296-308,
  * 360-419). spheres: per nucleus (centre xyz, radius, taper centre, taper width). */
 int cdftb_geometry_node_fields(int n_atoms, const double* charges, const double* positions, const double* spheres,
