@@ -285,10 +285,13 @@ class KohnShamStep:
         band = (occupations[0] * eigen.eigenvalues).sum()
         ham = self._bare
         phi = eigen.eigenvectors.to(torch.float64)
-        kinetic = ham.kinetic_energy_tensor(phi, occupations[0])
+        # <phi|T|phi> and the direct external energy take the same two integrals of sum_i f_i phi_i^2 (rho_out)
+        cross, potential = self.quadrature.external_energy_parts(rho_out, self.factor)
+        form = ham.measure.inner(phi, ham.kinetic_apply(phi))
+        kinetic = (occupations[0].to(torch.float64) * form).sum() - cross - potential
         dc_out = row_sums((p_in.effective * self.quadrature.mass_weights * rho_out)[None])[0]
         kinetic_plus_external = band - dc_out
-        external_direct = ham.external_energy_direct_tensor(rho_out)
+        external_direct = cross + 2.0 * potential
         harris = band - p_in.hartree_energy - p_in.xc_double_counting + p_in.xc_energy + self.ion_ion
         if p_out is None:
             total = harris
