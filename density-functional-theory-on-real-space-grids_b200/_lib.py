@@ -149,6 +149,10 @@ SIGNATURES: dict[str, tuple] = {
                                            c_void_p]),
     "cdftb_geometry_face_weights": (c_int, [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_double, c_double, c_double,
                                             c_double, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "cdftb_ritz_work_bytes": (c_int64, [c_int, c_int64]),
+    "cdftb_ritz_basis_f64": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_void_p, c_void_p, c_int64, c_void_p]),
+    "cdftb_ritz_vectors_f64": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_void_p, c_void_p,
+                                       c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
     "cdftb_geometry_sphere_nodes": (c_int, [c_int, c_int, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                             c_void_p]),
     "cdftb_geometry_node_fields": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_double, c_void_p, c_void_p, c_void_p,

@@ -8,6 +8,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace cdftb {
@@ -462,6 +464,34 @@ int ritz_chunks(int64_t n, int groups) {
     return static_cast<int>(chunks < 1 ? 1 : chunks);
 }
 
+// max that keeps a NaN, as torch's does.
+__device__ __forceinline__ double max_or_nan(double a, double b) { return isnan(a) || !(b >= a || isnan(b)) ? a : b; }
+
+// What an eigensolver iteration reads back, by one thread: residuals sqrt(max(|rho|^2, 0)); summary = worst
+// wanted residual, drift of the wanted values, orthonormality error max |V^T Q V - 1|, the top value, the
+// Cholesky status. It stands for a dozen elementwise and reduction launches over at most 64 numbers.
+__global__ void ritz_summary_kernel(const double* __restrict__ g2, const double* __restrict__ norms_sq,
+                                    const double* __restrict__ evals, const double* __restrict__ previous,
+                                    const int* __restrict__ info, int m, int n_states, double* __restrict__ residuals,
+                                    double* __restrict__ summary) {
+    double worst = 0.0, drift = 0.0, orth = 0.0;
+    for (int i = 0; i < m; ++i) {
+        const double sq = norms_sq[i];
+        const double r = sqrt(sq < 0.0 ? 0.0 : sq);
+        residuals[i] = r;
+        if (i < n_states) {
+            worst = max_or_nan(worst, r);
+            drift = max_or_nan(drift, fabs(evals[i] - previous[i]));
+        }
+        for (int j = 0; j < m; ++j) orth = max_or_nan(orth, fabs(g2[i * m + j] - (i == j ? 1.0 : 0.0)));
+    }
+    summary[0] = worst;
+    summary[1] = drift;
+    summary[2] = orth;
+    summary[3] = evals[m - 1];
+    summary[4] = info[0];
+}
+
 // CTAs along the points of each group: about 8 per SM over the whole launch (all groups), so that
 // with many groups every thread loops over several points instead of the launch running many
 // short waves of one point per thread.
@@ -601,3 +631,65 @@ extern "C" int cdftb_block_ritz_f64(const double* r, const double* basis, const 
     return check_launch();
 }
 
+
+namespace {
+
+// One iteration's small matrices, in the caller's work: Gram, L, subspace matrix, rotation, V^T Q V, |rho|^2,
+// the Cholesky status, then the scratch of the products and of the residual sums.
+struct RitzWork {
+    double *gram, *lower, *sub, *rot, *g2, *norms_sq;
+    int* info;
+    void* scratch;
+};
+
+int64_t ritz_scratch_bytes(int m, int64_t n) {
+    return std::max(cdftb_measure_cross_scratch_bytes(m, m, n, 1), cdftb_block_ritz_scratch_bytes(m, n, 1));
+}
+
+RitzWork ritz_work(void* work, int m) {
+    double* w = static_cast<double*>(work);
+    const int mm = m * m;
+    return {w, w + mm, w + 2 * mm, w + 3 * mm, w + 4 * mm, w + 5 * mm, reinterpret_cast<int*>(w + 5 * mm + m),
+            w + 5 * mm + m + 1};
+}
+
+}  // namespace
+
+extern "C" int64_t cdftb_ritz_work_bytes(int m, int64_t n) {
+    if (m <= 0 || m > 8 || n <= 0) return 0;
+    return (5 * m * m + m + 1) * int64_t(8) + ritz_scratch_bytes(m, n);
+}
+
+extern "C" int cdftb_ritz_basis_f64(const double* block, const double* q, int m, int64_t n, double* basis, void* work,
+                                    int64_t work_bytes, cdftb_stream_t stream) {
+    if (!block || !q || !basis || m <= 0 || m > 8 || n <= 0 || !work || work_bytes < cdftb_ritz_work_bytes(m, n))
+        return CDFTB_ERR_ARGUMENT;
+    const RitzWork w = ritz_work(work, m);
+    const int64_t stride = m * n;
+    int st = cdftb_measure_cross_f64(block, m, stride, block, m, stride, q, n, 1, w.gram, w.scratch,
+                                     ritz_scratch_bytes(m, n), stream);
+    if (st == CDFTB_OK) st = cdftb_small_cholesky_f64(w.gram, w.lower, w.info, m, 1, stream);
+    if (st != CDFTB_OK) return st;
+    return cdftb_block_trsm_lower_f64(w.lower, block, stride, basis, CDFTB_F64, stride, m, n, 1, stream);
+}
+
+extern "C" int cdftb_ritz_vectors_f64(const double* basis, const double* applied, const double* q, const double* previous,
+                                      int n_states, int m, int64_t n, double* vectors, double* evals, double* residuals,
+                                      double* summary, void* work, int64_t work_bytes, cdftb_stream_t stream) {
+    if (!basis || !applied || !q || !previous || !vectors || !evals || !residuals || !summary || m <= 0 || m > 8 ||
+        n <= 0 || n_states < 1 || n_states > m || !work || work_bytes < cdftb_ritz_work_bytes(m, n))
+        return CDFTB_ERR_ARGUMENT;
+    const RitzWork w = ritz_work(work, m);
+    const int64_t stride = m * n, scratch = ritz_scratch_bytes(m, n);
+    int st = cdftb_measure_cross_f64(basis, m, stride, applied, m, stride, q, n, 1, w.sub, w.scratch, scratch, stream);
+    if (st == CDFTB_OK) st = cdftb_small_eigh_f64(w.sub, evals, w.rot, m, 1, stream);
+    if (st == CDFTB_OK)
+        st = cdftb_block_ritz_f64(w.rot, basis, applied, evals, q, 0, m, n, 1, vectors, w.norms_sq, w.scratch, scratch,
+                                  stream);
+    if (st == CDFTB_OK)
+        st = cdftb_measure_cross_f64(vectors, m, stride, vectors, m, stride, q, n, 1, w.g2, w.scratch, scratch, stream);
+    if (st != CDFTB_OK) return st;
+    ritz_summary_kernel<<<1, 1, 0, as_stream(stream)>>>(w.g2, w.norms_sq, evals, previous, w.info, m, n_states, residuals,
+                                                        summary);
+    return check_launch();
+}

@@ -224,6 +224,19 @@ int cdftb_block_ritz_f64(const double* r, const double* basis, const double* app
                          const double* q, int64_t q_group_stride, int m, int64_t n, int groups, double* vectors,
                          double* norms_sq, void* scratch, int64_t scratch_bytes, cdftb_stream_t stream);
 
+/* One Rayleigh--Ritz step of an eigensolver iteration for a float64 block of m <= 8 orbitals around the
+ * caller's apply (rayleigh_ritz.py:51-115): basis = L^{-1} block with L L^T its Gram matrix in the measure,
+ * then, from applied = A basis, the Ritz values and vectors, the residual norms |A v - eps v| and, for
+ * the host, summary = { largest of the first n_states residuals, largest |evals - previous| of them,
+ * max |V^T Q V - 1|, the top Ritz value, the Cholesky status }. The steps are the entry points above; the
+ * two calls share work (cdftb_ritz_work_bytes, 8-byte aligned), which holds L and its status between. */
+int64_t cdftb_ritz_work_bytes(int m, int64_t n);
+int cdftb_ritz_basis_f64(const double* block, const double* q, int m, int64_t n, double* basis, void* work,
+                         int64_t work_bytes, cdftb_stream_t stream);
+int cdftb_ritz_vectors_f64(const double* basis, const double* applied, const double* q, const double* previous,
+                           int n_states, int m, int64_t n, double* vectors, double* evals, double* residuals,
+                           double* summary, void* work, int64_t work_bytes, cdftb_stream_t stream);
+
 /* (e5) out[g][i][p] = a[g][i][p] - evals[g][i] * b[g][i][p] (rayleigh_ritz.py:114 residual).
  * Each group's m rows are m consecutive rows of n elements, groups group_stride elements apart. */
 int cdftb_block_residual_f64(const double* a, const double* b, const double* evals, double* out, int m,
