@@ -131,6 +131,12 @@ SIGNATURES: dict[str, tuple] = {
                                                c_int, c_int64, c_void_p, c_int, c_int64, c_void_p, c_int64, c_void_p,
                                                c_int64, c_void_p]),
     "cdftb_cusp_coefficients_f64": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p]),
+    "cdftb_cusp_coefficients_density_f64": (c_int, [c_void_p] * 6 + [c_int] * 5 + [c_void_p] * 2),
+    "cdftb_potentials_lda_work_bytes": (c_int64, [c_int64, c_int64, c_int]),
+    "cdftb_potentials_node_lda_sums_f64": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
+                                                   c_int, c_int, c_void_p, c_void_p, c_int64, c_void_p]),
+    "cdftb_potentials_grid_lda_sums_f64": (c_int, [c_void_p] * 8 + [c_int, c_void_p, c_int64, c_int64, c_int]
+                                           + [c_void_p] * 5 + [c_int64, c_void_p]),
     "cdftb_hartree_split_f64": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int, c_void_p,
                                         c_void_p, c_void_p]),
     "cdftb_potentials_node_lda_f64": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,

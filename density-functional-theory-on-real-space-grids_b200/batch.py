@@ -574,27 +574,26 @@ class BatchedKohnShamStep:
         fields = torch.empty((2, b, n), **f)  # [rho | v_smooth]
         rho = fields[0]
         n_smooth = torch.empty((b, n), **f)
-        call("cdftb_hartree_split_f64", ptr(n_grid), ptr(self.f2), None, None, 0, n, b, ptr(rho), ptr(n_smooth), stream)
-        rho_nuc = torch.empty((b, na), **f)
-        call("cdftb_quadrature_interpolate_f64", ptr(g.step.nuclei_base), ptr(g.step.nuclei_w1d), na, *grid.shape,
-             ptr(rho), b, n, ptr(rho_nuc), na, stream)
         coef = torch.empty((b, na), **f)
-        call("cdftb_cusp_coefficients_f64", ptr(rho_nuc), ptr(g.step.nucleus_f2), ptr(g.step.overlap), na, b,
-             ptr(coef), stream)
+        call("cdftb_cusp_coefficients_density_f64", ptr(n_grid), ptr(self.f2), ptr(g.step.nuclei_base),
+             ptr(g.step.nuclei_w1d), ptr(g.step.nucleus_f2), ptr(g.step.overlap), na, *grid.shape, b, ptr(coef), stream)
         if v_smooth is None:
             call("cdftb_hartree_split_f64", ptr(n_grid), ptr(self.f2), ptr(g.step.cusp_grid), ptr(coef), na, n, b,
                  ptr(rho), ptr(n_smooth), stream)
             self.poisson.solve_batch(n_smooth, out=fields[1])
         else:
+            call("cdftb_hartree_split_f64", ptr(n_grid), ptr(self.f2), None, None, 0, n, b, ptr(rho), ptr(n_smooth),
+                 stream)
             fields[1].copy_(v_smooth)
         if node is None:
             node = q._interp_raw(fields.reshape(2 * b, n), 2 * b).reshape(2, b, m)
         else:
             node = node.contiguous()
         lift_in = torch.empty((b, 2, m), **f)
-        e_w = torch.empty((b, m), **f)
-        call("cdftb_potentials_node_lda_f64", ptr(node), m, ptr(q.weights), ptr(q.f2), ptr(g.step.v1s_node),
-             ptr(coef), na, b, ptr(lift_in), ptr(e_w), stream)
+        nbytes = _lib.library().cdftb_potentials_lda_work_bytes(m, n, b)
+        work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        call("cdftb_potentials_node_lda_sums_f64", ptr(node), m, n, ptr(q.weights), ptr(q.f2), ptr(g.step.v1s_node),
+             ptr(coef), na, b, ptr(lift_in), ptr(work), nbytes, stream)
         if lifted_h is None:
             lifted = q._lift_raw(lift_in, 2 * b).reshape(b, 2, n)
         else:
@@ -603,14 +602,13 @@ class BatchedKohnShamStep:
             lifted[:, 1] = q._lift_raw(lift_in[:, 1].contiguous(), b)
         effective = torch.empty((b, n), **f)
         v_hartree = torch.empty((b, n), **f)
-        terms = torch.empty((b, 3, n), **f)
-        call("cdftb_potentials_grid_lda_f64", ptr(n_grid), ptr(rho), ptr(self.f2), ptr(q.far_weights),
-             ptr(q.mass_weights), ptr(fields[1]), ptr(g.step.v1s_grid), ptr(coef), na, ptr(lifted), n, b,
-             ptr(effective), ptr(v_hartree), ptr(terms), None, stream)
-        sums = row_sums(terms)  # (b, 3)
-        node_sum = row_sums(e_w)  # (b,)
-        return BatchedPotentials(effective=effective, v_hartree=v_hartree, hartree_energy=0.5 * sums[:, 0],
-                                 xc_energy=node_sum + sums[:, 2], xc_double_counting=sums[:, 1], v_smooth=fields[1],
+        energies = torch.empty((b, 3), **f)
+        call("cdftb_potentials_grid_lda_sums_f64", ptr(n_grid), ptr(rho), ptr(self.f2), ptr(q.far_weights),
+             ptr(q.mass_weights), ptr(fields[1]), ptr(g.step.v1s_grid), ptr(coef), na, ptr(lifted), m, n, b,
+             ptr(effective), ptr(v_hartree), None, ptr(energies), ptr(work), nbytes, stream)
+        hartree_energy, xc_double_counting, xc_energy = energies.unbind(dim=1)
+        return BatchedPotentials(effective=effective, v_hartree=v_hartree, hartree_energy=hartree_energy,
+                                 xc_energy=xc_energy, xc_double_counting=xc_double_counting, v_smooth=fields[1],
                                  node=node, lifted_h=lifted[:, 0])
 
     def _potentials_generic(self, density: torch.Tensor) -> BatchedPotentials:

@@ -53,16 +53,13 @@ __global__ void xc_pbe_kernel(const double* __restrict__ n, const double* __rest
 }
 
 // c = S^{-1} (nucleus_f2 * rho(R_a)) by Gaussian elimination with partial pivoting, one system per
-// thread (step.py:240-242; n_atoms <= MAX_ATOMS).
-__global__ void cusp_coefficients_kernel(const double* __restrict__ rho_at_nuclei, const double* __restrict__ nucleus_f2,
-                                         const double* __restrict__ overlap, int na, int batch,
-                                         double* __restrict__ coef) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= batch) return;
+// thread (step.py:240-242; n_atoms <= MAX_ATOMS). rho_at_nuclei and coef: the system's own na values.
+__device__ void solve_cusp_coefficients(const double* rho_at_nuclei, const double* __restrict__ nucleus_f2,
+                                        const double* __restrict__ overlap, int na, double* coef) {
     double a[MAX_ATOMS][MAX_ATOMS + 1];
     for (int i = 0; i < na; ++i) {
         for (int j = 0; j < na; ++j) a[i][j] = overlap[i * na + j];
-        a[i][na] = nucleus_f2[i] * rho_at_nuclei[g * na + i];
+        a[i][na] = nucleus_f2[i] * rho_at_nuclei[i];
     }
     for (int c = 0; c < na; ++c) {
         int piv = c;
@@ -81,9 +78,48 @@ __global__ void cusp_coefficients_kernel(const double* __restrict__ rho_at_nucle
     }
     for (int r = na - 1; r >= 0; --r) {
         double v = a[r][na];
-        for (int k = r + 1; k < na; ++k) v -= a[r][k] * coef[g * na + k];
-        coef[g * na + r] = v / a[r][r];
+        for (int k = r + 1; k < na; ++k) v -= a[r][k] * coef[k];
+        coef[r] = v / a[r][r];
     }
+}
+
+__global__ void cusp_coefficients_kernel(const double* __restrict__ rho_at_nuclei, const double* __restrict__ nucleus_f2,
+                                         const double* __restrict__ overlap, int na, int batch,
+                                         double* __restrict__ coef) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < batch)
+        solve_cusp_coefficients(rho_at_nuclei + int64_t(g) * na, nucleus_f2, overlap, na, coef + int64_t(g) * na);
+}
+
+// The same from the density: rho(R_a) = L_a (n / f^2) over the 8^3 points around each nucleus, a CTA per
+// system, two points per thread. Only these 512 quotients are needed: forming rho on the grid first, to
+// interpolate it, took a pass over all points (32 systems at 65^3: 60 us for the three launches; this
+// kernel 5 us).
+__global__ void __launch_bounds__(256) cusp_coefficients_density_kernel(
+    const double* __restrict__ n, const double* __restrict__ f2, const int* __restrict__ base,
+    const double* __restrict__ w1d, const double* __restrict__ nucleus_f2, const double* __restrict__ overlap, int na,
+    int64_t np, int ny, int nz, double* __restrict__ coef) {
+    __shared__ double red[8][MAX_ATOMS], rho[MAX_ATOMS];
+    const int64_t g = blockIdx.x;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int a = t >> 6, b = (t >> 3) & 7, c = t & 7;  // taps (a and a + 4, b, c)
+    for (int k = 0; k < na; ++k) {
+        const double* w = w1d + k * 24;
+        const int64_t bx = base[k * 3] - 3 + a, by = base[k * 3 + 1] - 3 + b, bz = base[k * 3 + 2] - 3 + c;
+        const int64_t i0 = (bx * ny + by) * nz + bz, i1 = i0 + 4 * int64_t(ny) * nz;
+        double v = (w[8 + b] * w[16 + c]) * fma(w[a], n[g * np + i0] / f2[i0], w[a + 4] * (n[g * np + i1] / f2[i1]));
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if (lane == 0) red[warp][k] = v;
+    }
+    __syncthreads();
+    if (t < na) {
+        double v = 0.0;
+        for (int w = 0; w < 8; ++w) v += red[w][t];
+        rho[t] = v;
+    }
+    __syncthreads();
+    if (t == 0) solve_cusp_coefficients(rho, nucleus_f2, overlap, na, coef + g * na);
 }
 
 // rho = n / f^2 and n_smooth = n - sum_a c_a exp(-2 Z_a s_a) (step.py:235-244).
@@ -105,10 +141,30 @@ __global__ void hartree_split_kernel(const double* __restrict__ n, const double*
     }
 }
 
-// Node side of potentials(), LDA: x_H = w f2 vH, x_xc = w f2 v_xc (the lift inputs of the lumped
-// Hartree and XC weights) and e_w = w e_xc (the node part of the XC energy).
-// fields: rho_node (batch x m) followed by vsmooth_node (batch x m); outputs x [batch][2][m],
-// e_w [batch][m].
+// Node side of potentials(), LDA, at node i of system g: x_H = w f2 vH, x_xc = w f2 v_xc (the lift inputs
+// of the lumped Hartree and XC weights, x [batch][2][m]); returns e_w = w e_xc (the node part of the XC
+// energy). fields: rho_node (batch x m) followed by vsmooth_node (batch x m).
+__device__ __forceinline__ double node_lda(const double* __restrict__ fields, int64_t m,
+                                           const double* __restrict__ weights, const double* __restrict__ f2n,
+                                           const double* __restrict__ v1s_node, const double* __restrict__ coef, int na,
+                                           int batch, int64_t g, int64_t i, double* __restrict__ x) {
+    const double rho_node = fields[g * m + i];
+    double vh = 0.0;
+    for (int a = 0; a < na; ++a) {
+        const double t = coef[g * na + a] * v1s_node[a * m + i];
+        vh = (a == 0) ? t : vh + t;
+    }
+    vh = vh + fields[(batch + g) * m + i];
+    const double f2 = f2n[i];
+    const double nn = f2 * rho_node;
+    double e, v;
+    xc::lda_vwn(nn, e, v);
+    const double w = weights[i];
+    x[g * 2 * m + i] = w * (f2 * vh);
+    x[g * 2 * m + m + i] = w * (f2 * v);
+    return w * e;
+}
+
 __global__ void node_lda_kernel(const double* __restrict__ fields, int64_t m, const double* __restrict__ weights,
                                 const double* __restrict__ f2n, const double* __restrict__ v1s_node,
                                 const double* __restrict__ coef, int na, int batch, double* __restrict__ x,
@@ -117,56 +173,127 @@ __global__ void node_lda_kernel(const double* __restrict__ fields, int64_t m, co
     GRID_STRIDE(k, m * batch) {
         int64_t g, i;
         split_index(k, m, narrow, g, i);
-        const double rho_node = fields[g * m + i];
-        double vh = 0.0;
-        for (int a = 0; a < na; ++a) {
-            const double t = coef[g * na + a] * v1s_node[a * m + i];
-            vh = (a == 0) ? t : vh + t;
-        }
-        vh = vh + fields[(batch + g) * m + i];
-        const double f2 = f2n[i];
-        const double nn = f2 * rho_node;
-        double e, v;
-        xc::lda_vwn(nn, e, v);
-        const double w = weights[i];
-        x[g * 2 * m + i] = w * (f2 * vh);
-        x[g * 2 * m + m + i] = w * (f2 * v);
-        e_w[g * m + i] = w * e;
+        e_w[g * m + i] = node_lda(fields, m, weights, f2n, v1s_node, coef, na, batch, g, i, x);
     }
 }
 
-// Grid side, LDA: hartree_w = L_H + far_w (f2 vH), xc_w = L_xc + far_w (f2 v_xc),
-// effective = (hartree_w + xc_w) / omega (step.py:249-303); terms [3][np] = (hartree_w rho,
-// xc_w rho, far_w e_xc) for the energy sums; v_hartree = sum_a c_a v1s_a + v_smooth.
-__global__ void grid_lda_kernel(const double* __restrict__ n, const double* __restrict__ rho,
-                                const double* __restrict__ f2, const double* __restrict__ far_w,
-                                const double* __restrict__ mass, const double* __restrict__ v_smooth,
-                                const double* __restrict__ v1s_grid, const double* __restrict__ coef, int na,
-                                const double* __restrict__ lifted, int64_t np, int batch, double* __restrict__ effective,
-                                double* __restrict__ v_hartree, double* __restrict__ terms, double* __restrict__ v_xc) {
-    const bool narrow = np * batch <= 0xffffffffll;
-    GRID_STRIDE(k, np * batch) {
+// Grid side, LDA, at point i of system g: hartree_w = L_H + far_w (f2 vH), xc_w = L_xc + far_w (f2 v_xc),
+// effective = (hartree_w + xc_w) / omega (step.py:249-303); terms = (hartree_w rho, xc_w rho,
+// far_w e_xc) for the energy sums; v_hartree = sum_a c_a v1s_a + v_smooth.
+struct GridLda {
+    const double *n, *rho, *f2, *far_w, *mass, *v_smooth, *v1s_grid, *coef;
+    int na;
+    const double* lifted;
+    int64_t np;
+    double *effective, *v_hartree, *v_xc;
+};
+
+__device__ __forceinline__ void grid_lda(const GridLda& p, int64_t g, int64_t i, double terms[3]) {
+    const int64_t np = p.np, k = g * np + i;
+    double vh = 0.0;
+    for (int a = 0; a < p.na; ++a) {
+        const double t = p.coef[g * p.na + a] * p.v1s_grid[a * np + i];
+        vh = (a == 0) ? t : vh + t;
+    }
+    vh = vh + p.v_smooth[k];
+    double e, v;
+    xc::lda_vwn(p.n[k], e, v);
+    const double fw = p.far_w[i];
+    const double f = p.f2[i];
+    const double hw = p.lifted[g * 2 * np + i] + fw * (f * vh);
+    const double xw = p.lifted[g * 2 * np + np + i] + fw * (f * v);
+    const double r = p.rho[k];
+    p.effective[k] = (hw + xw) / p.mass[i];
+    p.v_hartree[k] = vh;
+    if (p.v_xc) p.v_xc[k] = v;
+    terms[0] = hw * r;
+    terms[1] = xw * r;
+    terms[2] = fw * e;
+}
+
+__global__ void grid_lda_kernel(const GridLda p, int batch, double* __restrict__ terms) {
+    const bool narrow = p.np * batch <= 0xffffffffll;
+    GRID_STRIDE(k, p.np * batch) {
         int64_t g, i;
-        split_index(k, np, narrow, g, i);
-        double vh = 0.0;
-        for (int a = 0; a < na; ++a) {
-            const double t = coef[g * na + a] * v1s_grid[a * np + i];
-            vh = (a == 0) ? t : vh + t;
-        }
-        vh = vh + v_smooth[k];
-        double e, v;
-        xc::lda_vwn(n[k], e, v);
-        const double fw = far_w[i];
-        const double f = f2[i];
-        const double hw = lifted[g * 2 * np + i] + fw * (f * vh);
-        const double xw = lifted[g * 2 * np + np + i] + fw * (f * v);
-        const double r = rho[k];
-        effective[k] = (hw + xw) / mass[i];
-        v_hartree[k] = vh;
-        if (v_xc) v_xc[k] = v;
-        terms[g * 3 * np + i] = hw * r;
-        terms[g * 3 * np + np + i] = xw * r;
-        terms[g * 3 * np + 2 * np + i] = fw * e;
+        split_index(k, p.np, narrow, g, i);
+        double t[3];
+        grid_lda(p, g, i, t);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) terms[(g * 3 + j) * p.np + i] = t[j];
+    }
+}
+
+// Both sides with their energy sums: a CTA takes sum_points points of one system and leaves one partial
+// per sum, lda_energies_kernel adds a system's partials in order. The terms never reach memory, where
+// writing them and summing the rows took 48 of a point's 112 bytes; what is left is bound by the FP64 issue
+// of the functional (32 systems at 65^3: 196 us with the sums, 193 and 50 us apart).
+constexpr int kSumThreads = 256;
+
+// Points of a CTA: one per thread until the launch has 16 CTAs per SM, then up to 8 (the sums over the
+// block and the partials are then a small part).
+int64_t sum_points(int64_t n, int64_t batch) {
+    const int64_t k = n * batch / (int64_t(kSumThreads) * 148 * 16);
+    return kSumThreads * (k < 1 ? 1 : k > 8 ? 8 : k);
+}
+
+template <int N>
+__device__ __forceinline__ void block_sums(double v[N], double* sums) {
+    __shared__ double red[kSumThreads / 32][N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v[j] += __shfl_down_sync(0xffffffffu, v[j], off);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][j] = v[j];
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double t = 0.0;
+        for (int w = 0; w < kSumThreads / 32; ++w) t += red[w][threadIdx.x];
+        sums[threadIdx.x] = t;
+    }
+}
+
+__global__ void __launch_bounds__(kSumThreads) node_lda_sums_kernel(
+    const double* __restrict__ fields, int64_t m, int64_t points, int64_t chunks, const double* __restrict__ weights,
+    const double* __restrict__ f2n, const double* __restrict__ v1s_node, const double* __restrict__ coef, int na,
+    int batch, double* __restrict__ x, double* __restrict__ partial) {
+    const int64_t g = blockIdx.x / chunks, i0 = (blockIdx.x - g * chunks) * points;
+    double sum[1] = {0.0};
+    for (int64_t i = i0 + threadIdx.x; i < i0 + points && i < m; i += kSumThreads)
+        sum[0] += node_lda(fields, m, weights, f2n, v1s_node, coef, na, batch, g, i, x);
+    block_sums<1>(sum, partial + blockIdx.x);
+}
+
+__global__ void __launch_bounds__(kSumThreads) grid_lda_sums_kernel(const GridLda p, int64_t points, int64_t chunks,
+                                                                    double* __restrict__ partial) {
+    const int64_t g = blockIdx.x / chunks, i0 = (blockIdx.x - g * chunks) * points;
+    double sum[3] = {0.0, 0.0, 0.0};
+    for (int64_t i = i0 + threadIdx.x; i < i0 + points && i < p.np; i += kSumThreads) {
+        double t[3];
+        grid_lda(p, g, i, t);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) sum[j] += t[j];
+    }
+    block_sums<3>(sum, partial + int64_t(blockIdx.x) * 3);
+}
+
+// energies [batch][3] = (Hartree energy, XC double counting, XC energy), a CTA per system.
+__global__ void __launch_bounds__(kSumThreads) lda_energies_kernel(const double* __restrict__ node, int64_t node_chunks,
+                                                                   const double* __restrict__ grid, int64_t grid_chunks,
+                                                                   double* __restrict__ energies) {
+    __shared__ double sums[4];
+    const int64_t g = blockIdx.x;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int64_t c = threadIdx.x; c < grid_chunks; c += kSumThreads)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) v[j] += grid[(g * grid_chunks + c) * 3 + j];
+    for (int64_t c = threadIdx.x; c < node_chunks; c += kSumThreads) v[3] += node[g * node_chunks + c];
+    block_sums<4>(v, sums);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        energies[g * 3] = 0.5 * sums[0];
+        energies[g * 3 + 1] = sums[1];
+        energies[g * 3 + 2] = sums[3] + sums[2];
     }
 }
 
@@ -405,9 +532,73 @@ extern "C" int cdftb_potentials_grid_lda_f64(const double* density, const double
     if (!density || !rho || !f2 || !far_weights || !mass_weights || !v_smooth || !lifted || !effective || !v_hartree ||
         !terms || (n_atoms > 0 && (!v1s_grid || !coefficients)))
         return CDFTB_ERR_ARGUMENT;
-    grid_lda_kernel<<<blocks_for(n_points * batch, 256), 256, 0, as_stream(stream)>>>(
-        density, rho, f2, far_weights, mass_weights, v_smooth, v1s_grid, coefficients, n_atoms, lifted, n_points, batch,
-        effective, v_hartree, terms, v_xc);
+    const GridLda p{density,  rho,     f2,     far_weights, mass_weights, v_smooth,  v1s_grid,
+                    coefficients, n_atoms, lifted, n_points,    effective,    v_hartree, v_xc};
+    grid_lda_kernel<<<blocks_for(n_points * batch, 256), 256, 0, as_stream(stream)>>>(p, batch, terms);
+    return check_launch();
+}
+
+extern "C" int cdftb_cusp_coefficients_density_f64(const double* density, const double* f2, const int* nuclei_base,
+                                                   const double* nuclei_w1d, const double* nucleus_f2,
+                                                   const double* overlap, int n_atoms, int nx, int ny, int nz, int batch,
+                                                   double* coefficients, cdftb_stream_t stream) {
+    if (n_atoms < 1 || n_atoms > MAX_ATOMS || batch < 1 || nx < 1 || ny < 1 || nz < 1 || !density || !f2 ||
+        !nuclei_base || !nuclei_w1d || !nucleus_f2 || !overlap || !coefficients)
+        return CDFTB_ERR_ARGUMENT;
+    cusp_coefficients_density_kernel<<<static_cast<unsigned>(batch), 256, 0, as_stream(stream)>>>(
+        density, f2, nuclei_base, nuclei_w1d, nucleus_f2, overlap, n_atoms, int64_t(nx) * ny * nz, ny, nz, coefficients);
+    return check_launch();
+}
+
+extern "C" int64_t cdftb_potentials_lda_work_bytes(int64_t m, int64_t n_points, int batch) {
+    if (m < 0 || n_points <= 0 || batch < 1) return 0;
+    return (ceil_div(m, sum_points(m, batch)) + 3 * ceil_div(n_points, sum_points(n_points, batch))) * batch * 8;
+}
+
+extern "C" int cdftb_potentials_node_lda_sums_f64(const double* fields, int64_t m, int64_t n_points,
+                                                  const double* weights, const double* f2_node, const double* v1s_node,
+                                                  const double* coefficients, int n_atoms, int batch,
+                                                  double* lift_inputs, void* work, int64_t work_bytes,
+                                                  cdftb_stream_t stream) {
+    if (m < 0 || n_points <= 0 || n_atoms < 0 || n_atoms > MAX_ATOMS || batch < 1 || !work ||
+        work_bytes < cdftb_potentials_lda_work_bytes(m, n_points, batch))
+        return CDFTB_ERR_ARGUMENT;
+    if (m == 0) return CDFTB_OK;
+    if (!fields || !weights || !f2_node || !lift_inputs || (n_atoms > 0 && (!v1s_node || !coefficients)))
+        return CDFTB_ERR_ARGUMENT;
+    const int64_t points = sum_points(m, batch), chunks = ceil_div(m, points);
+    if (chunks * batch > 0x7fffffffll) return CDFTB_ERR_CAPACITY;
+    node_lda_sums_kernel<<<static_cast<unsigned>(chunks * batch), kSumThreads, 0, as_stream(stream)>>>(
+        fields, m, points, chunks, weights, f2_node, v1s_node, coefficients, n_atoms, batch, lift_inputs,
+        static_cast<double*>(work));
+    return check_launch();
+}
+
+extern "C" int cdftb_potentials_grid_lda_sums_f64(const double* density, const double* rho, const double* f2,
+                                                  const double* far_weights, const double* mass_weights,
+                                                  const double* v_smooth, const double* v1s_grid,
+                                                  const double* coefficients, int n_atoms, const double* lifted,
+                                                  int64_t m, int64_t n_points, int batch, double* effective,
+                                                  double* v_hartree, double* v_xc, double* energies, void* work,
+                                                  int64_t work_bytes, cdftb_stream_t stream) {
+    if (m < 0 || n_points <= 0 || batch < 1 || n_atoms < 0 || n_atoms > MAX_ATOMS || !work ||
+        work_bytes < cdftb_potentials_lda_work_bytes(m, n_points, batch))
+        return CDFTB_ERR_ARGUMENT;
+    if (!density || !rho || !f2 || !far_weights || !mass_weights || !v_smooth || !lifted || !effective || !v_hartree ||
+        !energies || (n_atoms > 0 && (!v1s_grid || !coefficients)))
+        return CDFTB_ERR_ARGUMENT;
+    const int64_t node_chunks = ceil_div(m, sum_points(m, batch));
+    const int64_t points = sum_points(n_points, batch), chunks = ceil_div(n_points, points);
+    if (chunks * batch > 0x7fffffffll) return CDFTB_ERR_CAPACITY;
+    double* node = static_cast<double*>(work);
+    double* grid = node + node_chunks * batch;
+    const GridLda p{density,  rho,     f2,     far_weights, mass_weights, v_smooth,  v1s_grid,
+                    coefficients, n_atoms, lifted, n_points,    effective,    v_hartree, v_xc};
+    cudaStream_t s = as_stream(stream);
+    grid_lda_sums_kernel<<<static_cast<unsigned>(chunks * batch), kSumThreads, 0, s>>>(p, points, chunks, grid);
+    const int st = check_launch();
+    if (st != CDFTB_OK) return st;
+    lda_energies_kernel<<<static_cast<unsigned>(batch), kSumThreads, 0, s>>>(node, node_chunks, grid, chunks, energies);
     return check_launch();
 }
 

@@ -127,34 +127,29 @@ class KohnShamStep:
         fields = torch.empty((2, n), dtype=torch.float64, device=dev)  # [rho, v_smooth]
         rho = fields[0]
         n_smooth = self._scratch_n
-        call("cdftb_hartree_split_f64", ptr(n_grid), ptr(self._f2_grid), None, None, 0, n, 1, ptr(rho), ptr(n_smooth),
-             stream)
-        rho_nuc = torch.empty((1, na), dtype=torch.float64, device=dev)
-        call("cdftb_quadrature_interpolate_f64", ptr(g.step.nuclei_base), ptr(g.step.nuclei_w1d), na, *grid.shape,
-             ptr(rho), 1, n, ptr(rho_nuc), na, stream)
         coef = torch.empty(na, dtype=torch.float64, device=dev)
-        call("cdftb_cusp_coefficients_f64", ptr(rho_nuc), ptr(g.step.nucleus_f2), ptr(g.step.overlap), na, 1, ptr(coef),
-             stream)
+        call("cdftb_cusp_coefficients_density_f64", ptr(n_grid), ptr(self._f2_grid), ptr(g.step.nuclei_base),
+             ptr(g.step.nuclei_w1d), ptr(g.step.nucleus_f2), ptr(g.step.overlap), na, *grid.shape, 1, ptr(coef), stream)
         call("cdftb_hartree_split_f64", ptr(n_grid), ptr(self._f2_grid), ptr(g.step.cusp_grid), ptr(coef), na, n, 1,
              ptr(rho), ptr(n_smooth), stream)
         self.poisson.solve_batch(n_smooth.reshape(1, n), out=fields[1].reshape(1, n))
         node_fields = q._interp_raw(fields, 2)
         lift_in = torch.empty((2, m), dtype=torch.float64, device=dev)
-        e_w = torch.empty(m, dtype=torch.float64, device=dev)
-        call("cdftb_potentials_node_lda_f64", ptr(node_fields), m, ptr(q.weights), ptr(q.f2), ptr(g.step.v1s_node),
-             ptr(coef), na, 1, ptr(lift_in), ptr(e_w), stream)
+        nbytes = _lib.library().cdftb_potentials_lda_work_bytes(m, n, 1)
+        work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        call("cdftb_potentials_node_lda_sums_f64", ptr(node_fields), m, n, ptr(q.weights), ptr(q.f2),
+             ptr(g.step.v1s_node), ptr(coef), na, 1, ptr(lift_in), ptr(work), nbytes, stream)
         lifted = q._lift_raw(lift_in, 2)
         effective = torch.empty(n, dtype=torch.float64, device=dev)
         v_hartree = torch.empty(n, dtype=torch.float64, device=dev)
         v_xc = torch.empty(n, dtype=torch.float64, device=dev)
-        terms = torch.empty((3, n), dtype=torch.float64, device=dev)
-        call("cdftb_potentials_grid_lda_f64", ptr(n_grid), ptr(rho), ptr(self._f2_grid), ptr(q.far_weights),
-             ptr(q.mass_weights), ptr(fields[1]), ptr(g.step.v1s_grid), ptr(coef), na, ptr(lifted), n, 1,
-             ptr(effective), ptr(v_hartree), ptr(terms), ptr(v_xc), stream)
-        sums = row_sums(terms)
-        node_sum = row_sums(e_w.reshape(1, m))[0]
-        return Potentials(v_hartree=v_hartree, v_xc=v_xc[None, :], effective=effective, hartree_energy=0.5 * sums[0],
-                          xc_energy=node_sum + sums[2], xc_double_counting=sums[1], hartree_coefficients=coef)
+        energies = torch.empty(3, dtype=torch.float64, device=dev)
+        call("cdftb_potentials_grid_lda_sums_f64", ptr(n_grid), ptr(rho), ptr(self._f2_grid), ptr(q.far_weights),
+             ptr(q.mass_weights), ptr(fields[1]), ptr(g.step.v1s_grid), ptr(coef), na, ptr(lifted), m, n, 1,
+             ptr(effective), ptr(v_hartree), ptr(v_xc), ptr(energies), ptr(work), nbytes, stream)
+        hartree_energy, xc_double_counting, xc_energy = energies.unbind()
+        return Potentials(v_hartree=v_hartree, v_xc=v_xc[None, :], effective=effective, hartree_energy=hartree_energy,
+                          xc_energy=xc_energy, xc_double_counting=xc_double_counting, hartree_coefficients=coef)
 
     def _potentials_generic(self, density: torch.Tensor) -> Potentials:
         """Potentials for any native functional (step.py:224-313) through ``functional.evaluate``;

@@ -442,6 +442,27 @@ int cdftb_density_residual_f64(const double* vectors, const double* occupations,
 int cdftb_external_grid_terms_f64(const double* grad, const double* rho, const double* weight, const double* grad_u,
                                   const double* transformed_potential, const double* far_weights, int64_t n_points,
                                   int batch, double* out, cdftb_stream_t stream);
+/* The coefficients straight from the density: rho(R_a) interpolated from n / f^2 at the 8^3 points of each
+ * nucleus' stencil (nuclei_base (n_atoms, 3), nuclei_w1d (n_atoms, 24); step.py:235-242). */
+int cdftb_cusp_coefficients_density_f64(const double* density, const double* f2, const int* nuclei_base,
+                                        const double* nuclei_w1d, const double* nucleus_f2, const double* overlap,
+                                        int n_atoms, int nx, int ny, int nz, int batch, double* coefficients,
+                                        cdftb_stream_t stream);
+/* The node and grid sides of the LDA potentials as above with their energy sums formed on the way
+ * (step.py:249-303): the node call leaves partial sums of w e_xc in work (cdftb_potentials_lda_work_bytes),
+ * the grid call, given the same m, n_points, batch and work after it, adds them: energies [batch][3] =
+ * Hartree energy, XC double counting, XC energy. v_xc may be NULL. */
+int64_t cdftb_potentials_lda_work_bytes(int64_t m, int64_t n_points, int batch);
+int cdftb_potentials_node_lda_sums_f64(const double* fields, int64_t m, int64_t n_points, const double* weights,
+                                       const double* f2_node, const double* v1s_node, const double* coefficients,
+                                       int n_atoms, int batch, double* lift_inputs, void* work, int64_t work_bytes,
+                                       cdftb_stream_t stream);
+int cdftb_potentials_grid_lda_sums_f64(const double* density, const double* rho, const double* f2,
+                                       const double* far_weights, const double* mass_weights, const double* v_smooth,
+                                       const double* v1s_grid, const double* coefficients, int n_atoms,
+                                       const double* lifted, int64_t m, int64_t n_points, int batch, double* effective,
+                                       double* v_hartree, double* v_xc, double* energies, void* work,
+                                       int64_t work_bytes, cdftb_stream_t stream);
 /* Deterministic row sums of a rows x len array (the energy integrals). */
 int64_t cdftb_row_sums_scratch_bytes(int rows, int64_t len);
 int cdftb_row_sums_f64(const double* a, int rows, int64_t len, double* out, void* scratch, int64_t scratch_bytes,
