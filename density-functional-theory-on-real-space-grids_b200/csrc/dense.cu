@@ -464,6 +464,12 @@ int ritz_chunks(int64_t n, int groups) {
     return static_cast<int>(chunks < 1 ? 1 : chunks);
 }
 
+// beta = sqrt(max(<w,w>, 0)).
+__global__ void lanczos_beta_kernel(const double* __restrict__ wsq, double* __restrict__ beta) {
+    const double x = *wsq;
+    *beta = sqrt(x < 0.0 ? 0.0 : x);
+}
+
 // max that keeps a NaN, as torch's does.
 __device__ __forceinline__ double max_or_nan(double a, double b) { return isnan(a) || !(b >= a || isnan(b)) ? a : b; }
 
@@ -692,4 +698,86 @@ extern "C" int cdftb_ritz_vectors_f64(const double* basis, const double* applied
     ritz_summary_kernel<<<1, 1, 0, as_stream(stream)>>>(w.g2, w.norms_sq, evals, previous, w.info, m, n_states, residuals,
                                                         summary);
     return check_launch();
+}
+
+namespace {
+
+// The recurrence's vectors and scalars, the products' partials and the apply's scratch, each from a
+// 256-byte boundary of work.
+struct LanczosWork {
+    double *v, *v_prev, *w, *scalars;
+    void *cross, *apply;
+    int64_t cross_bytes, apply_bytes, total;
+};
+
+LanczosWork lanczos_work(const cdftb_operator* op, void* work) {
+    const int64_t n = int64_t(op->nx) * op->ny * op->nz;
+    LanczosWork l{};
+    l.cross_bytes = cdftb_measure_cross_scratch_bytes(1, 1, n, 1);
+    l.apply_bytes = cdftb_cusp_apply_work_bytes(op, 1);
+    char* base = static_cast<char*>(work);
+    int64_t at = 0;
+    auto take = [&](int64_t bytes) {
+        const int64_t here = at;
+        at += (bytes + 255) / 256 * 256;
+        return here;
+    };
+    const int64_t v = take(n * 8), v_prev = take(n * 8), w = take(n * 8), scalars = take(4 * 8);
+    const int64_t cross = take(l.cross_bytes), apply = take(l.apply_bytes);
+    l.total = at;
+    if (base) {
+        l.v = reinterpret_cast<double*>(base + v);
+        l.v_prev = reinterpret_cast<double*>(base + v_prev);
+        l.w = reinterpret_cast<double*>(base + w);
+        l.scalars = reinterpret_cast<double*>(base + scalars);
+        l.cross = base + cross;
+        l.apply = l.apply_bytes > 0 ? base + apply : nullptr;
+    }
+    return l;
+}
+
+}  // namespace
+
+extern "C" int64_t cdftb_lanczos_work_bytes(const cdftb_operator* op) {
+    if (!op || op->nx <= 0 || op->ny <= 0 || op->nz <= 0) return 0;
+    return lanczos_work(op, nullptr).total;
+}
+
+extern "C" int cdftb_lanczos_f64(const cdftb_operator* op, const double* q, const double* start, int steps, double* values,
+                                 void* work, int64_t work_bytes, cdftb_stream_t stream) {
+    if (!op || !q || !start || !values || steps < 1 || op->dtype != CDFTB_F64 || op->nx <= 0 || op->ny <= 0 ||
+        op->nz <= 0 || !work || reinterpret_cast<uintptr_t>(work) % 16 != 0 || work_bytes < cdftb_lanczos_work_bytes(op))
+        return CDFTB_ERR_ARGUMENT;
+    const int64_t n = int64_t(op->nx) * op->ny * op->nz;
+    LanczosWork l = lanczos_work(op, work);
+    cudaStream_t s = as_stream(stream);
+    double *zero = l.scalars, *wsq = zero + 1, *c1 = zero + 2, *c2 = zero + 3;
+    auto inner = [&](const double* a, const double* b, double* out) {
+        return cdftb_measure_cross_f64(a, 1, n, b, 1, n, q, n, 1, out, l.cross, l.cross_bytes, stream);
+    };
+    int st = check(cudaMemcpyAsync(l.v, start, n * 8, cudaMemcpyDeviceToDevice, s));
+    if (st == CDFTB_OK) st = check(cudaMemsetAsync(l.v_prev, 0, n * 8, s));
+    if (st == CDFTB_OK) st = check(cudaMemsetAsync(zero, 0, 8, s));
+    if (st == CDFTB_OK) st = inner(l.v, l.v, wsq);
+    if (st == CDFTB_OK) st = cdftb_lanczos_update_f64(2, l.v, nullptr, nullptr, wsq, nullptr, n, 1, stream);
+    for (int k = 0; k < steps && st == CDFTB_OK; ++k) {
+        double *alpha = values + k, *beta = values + steps + k;
+        st = cdftb_cusp_apply(op, l.v, CDFTB_F64, l.w, CDFTB_F64, 1, 0, l.apply, l.apply_bytes, stream);
+        if (st == CDFTB_OK) st = inner(l.v, l.w, alpha);
+        if (st == CDFTB_OK)
+            st = cdftb_lanczos_update_f64(0, l.w, l.v, l.v_prev, alpha, k == 0 ? zero : beta - 1, n, 1, stream);
+        if (st == CDFTB_OK) st = inner(l.w, l.v, c1);
+        if (st == CDFTB_OK) st = inner(l.w, l.v_prev, c2);
+        if (st == CDFTB_OK) st = cdftb_lanczos_update_f64(1, l.w, l.v, l.v_prev, c1, c2, n, 1, stream);
+        if (st == CDFTB_OK) st = inner(l.w, l.w, wsq);
+        if (st != CDFTB_OK) break;
+        lanczos_beta_kernel<<<1, 1, 0, s>>>(wsq, beta);
+        st = check_launch();
+        if (st == CDFTB_OK) st = cdftb_lanczos_update_f64(2, l.w, nullptr, nullptr, wsq, nullptr, n, 1, stream);
+        double* old = l.v_prev;  // v_prev, v, w <- v, w, the freed buffer
+        l.v_prev = l.v;
+        l.v = l.w;
+        l.w = old;
+    }
+    return st;
 }

@@ -271,13 +271,22 @@ def seeded_randn(shape, generator, *, device, dtype=torch.float64) -> torch.Tens
     return torch.randn(size, device=source, dtype=dtype, generator=generator).to(device)
 
 
-def lanczos_bounds(hamiltonian: CuspFactoredHamiltonian, start: torch.Tensor, steps: int, safety: float):
-    """The rigorous Lanczos enclosure (``src/cdft/operators/hamiltonian.py:29-89``).
+def _native_lanczos(hamiltonian: CuspFactoredHamiltonian, start: torch.Tensor, steps: int) -> torch.Tensor:
+    """``[alpha | beta]`` by one library call: a step's thirteen launches are issued from native code (0.9 ms for 12
+    steps at 33^3, paced by the device; from Python 1.9 ms)."""
+    op = hamiltonian.operator()
+    v = start.to(torch.float64).contiguous()
+    values = torch.empty(2 * steps, dtype=torch.float64, device=v.device)
+    nbytes = _lib.library().cdftb_lanczos_work_bytes(ctypes.byref(op))
+    work = torch.empty(nbytes, dtype=torch.uint8, device=v.device)
+    hamiltonian.note_applications(steps)
+    call("cdftb_lanczos_f64", ctypes.byref(op), ptr(hamiltonian.measure.quadrature), ptr(v), steps, ptr(values), ptr(work),
+         nbytes, stream_handle(v.device))
+    return values
 
-    Vectors, products and updates stay on the device (the recurrence scalars are device values
-    fed to the update kernel); alpha and beta are read once after the loop and the small
-    tridiagonal problem is solved on the host, as in the reference.
-    """
+
+def _lanczos_recurrence(hamiltonian, start: torch.Tensor, steps: int) -> torch.Tensor:
+    """The same for any operator with an ``apply``."""
     q = hamiltonian.measure.quadrature
     n = start.shape[-1]
     dev = start.device
@@ -303,7 +312,22 @@ def lanczos_bounds(hamiltonian: CuspFactoredHamiltonian, start: torch.Tensor, st
         call("cdftb_lanczos_update_f64", 2, ptr(w), None, None, ptr(wsq), None, n, 1, stream)
         v_prev, v = v, w
         beta_prev = beta
-    values = torch.cat([*alphas, *betas]).tolist()
+    return torch.cat([*alphas, *betas])
+
+
+def lanczos_bounds(hamiltonian: CuspFactoredHamiltonian, start: torch.Tensor, steps: int, safety: float):
+    """The rigorous Lanczos enclosure (``src/cdft/operators/hamiltonian.py:29-89``).
+
+    Vectors, products and updates stay on the device (the recurrence scalars are device values
+    fed to the update kernel); alpha and beta are read once after the loop and the small
+    tridiagonal problem is solved on the host, as in the reference.
+    """
+    if (type(hamiltonian) is CuspFactoredHamiltonian and hamiltonian.dtype == torch.float64 and steps >= 1
+            and start.device.type == "cuda" and start.numel() == hamiltonian.grid.n_points):
+        values = _native_lanczos(hamiltonian, start, steps)
+    else:
+        values = _lanczos_recurrence(hamiltonian, start, steps)
+    values = values.tolist()
     _lib.check_device_status("lanczos_bounds")
     a = values[:steps]
     b = values[steps:]

@@ -224,6 +224,13 @@ int cdftb_block_ritz_f64(const double* r, const double* basis, const double* app
                          const double* q, int64_t q_group_stride, int m, int64_t n, int groups, double* vectors,
                          double* norms_sq, void* scratch, int64_t scratch_bytes, cdftb_stream_t stream);
 
+/* The Lanczos recurrence of the spectral enclosure (src/cdft/operators/hamiltonian.py:29-89) for a float64
+ * operator, from start (n), by the apply, products and updates above: values[0..steps) = alpha,
+ * values[steps..2 steps) = beta, on the device. work: cdftb_lanczos_work_bytes, 16-byte aligned. */
+int64_t cdftb_lanczos_work_bytes(const cdftb_operator* op);
+int cdftb_lanczos_f64(const cdftb_operator* op, const double* q, const double* start, int steps, double* values,
+                      void* work, int64_t work_bytes, cdftb_stream_t stream);
+
 /* One Rayleigh--Ritz step of an eigensolver iteration for a float64 block of m <= 8 orbitals around the
  * caller's apply (rayleigh_ritz.py:51-115): basis = L^{-1} block with L L^T its Gram matrix in the measure,
  * then, from applied = A basis, the Ritz values and vectors, the residual norms |A v - eps v| and, for
