@@ -155,6 +155,8 @@ SIGNATURES: dict[str, tuple] = {
                                            c_void_p]),
     "cdftb_geometry_face_weights": (c_int, [c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_double, c_double, c_double,
                                             c_double, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "cdftb_cusp_apply_solved_f64": (c_int, [ctypes.POINTER(Operator), c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
+                                            c_void_p, c_int64, c_void_p]),
     "cdftb_lanczos_work_bytes": (c_int64, [ctypes.POINTER(Operator)]),
     "cdftb_lanczos_f64": (c_int, [ctypes.POINTER(Operator), c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int64,
                                   c_void_p]),

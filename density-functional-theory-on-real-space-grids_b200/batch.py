@@ -95,6 +95,17 @@ class BatchedHamiltonian:
             self.applications += 1
         return out
 
+    def apply_solved(self, lower: torch.Tensor, block: torch.Tensor, basis: torch.Tensor) -> torch.Tensor:
+        """``basis = L^-1 block`` per system and ``A basis`` (float64), the basis packed as it is formed."""
+        b, k, _ = block.shape
+        out = torch.empty_like(block)
+        op = self._op(k)
+        work = apply_workspace(op, b * k, block.device)
+        call("cdftb_cusp_apply_solved_f64", ctypes.byref(op), ptr(lower), ptr(block), ptr(basis), ptr(out), b * k,
+             ptr(work), work.numel(), stream_handle(block.device))
+        self.applications += 1
+        return out
+
     def filter(self, block: torch.Tensor, table: torch.Tensor, degree: int) -> torch.Tensor:
         """The fused Chebyshev filter on ``(B, k, N)`` float64 blocks, one coefficient table per system."""
         x = block.contiguous()
@@ -220,8 +231,11 @@ def batched_rayleigh_ritz(h: BatchedHamiltonian, block: torch.Tensor, check_orth
     rb = _RB.get(b, m, dev)
     call("cdftb_small_cholesky_f64", ptr(gram), ptr(rb.lower), ptr(rb.info), m, b, stream)
     basis = torch.empty_like(flat)
-    call("cdftb_block_trsm_lower_f64", ptr(rb.lower), ptr(flat), m * n, ptr(basis), F64, m * n, m, n, b, stream)
-    applied = h.apply(basis)
+    if type(h) is BatchedHamiltonian and h.dtype == torch.float64:
+        applied = h.apply_solved(rb.lower, flat, basis)
+    else:
+        call("cdftb_block_trsm_lower_f64", ptr(rb.lower), ptr(flat), m * n, ptr(basis), F64, m * n, m, n, b, stream)
+        applied = h.apply(basis)
     sub = measure_cross(basis, applied, q, b)
     call("cdftb_small_eigh_f64", ptr(sub), ptr(rb.evals), ptr(rb.rot), m, b, stream)
     vectors = torch.empty_like(flat)

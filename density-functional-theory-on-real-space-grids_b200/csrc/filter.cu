@@ -1416,6 +1416,82 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(const __grid_constan
     }
 }
 
+// The columns' triangular solve x = L^{-1} b of each group (as trsm_lower_fixed_kernel, bit for bit) that
+// leaves the basis in caller layout and in float64 wide lanes: the block is read once and the basis not
+// read again to be packed. HBM bounds it (3 M values per point and group). A thread takes a point of P
+// groups, so that P M orbitals fill whole lanes. 32 groups of 5 at 65^3: 170 us (HBM at its copy rate: 161), where the solve and
+// the packing took 136 and 100.
+template <int M>
+struct SolveShape {
+    static constexpr int P = M % 2 ? 2 : 1, LANES = P * M / 2;
+};
+
+template <int M>
+__global__ void __launch_bounds__(256) solve_pack_kernel(const double* __restrict__ lower, const double* __restrict__ in,
+                                                         int groups, int64_t n, int64_t per_lane, int nz, int nzp,
+                                                         int64_t lane_total, double* __restrict__ basis,
+                                                         double2* __restrict__ lanes) {
+    constexpr int P = SolveShape<M>::P, LANES = SolveShape<M>::LANES;
+    __shared__ double l[P * M * M];
+    const int g0 = blockIdx.y * P;
+    for (int i = threadIdx.x; i < P * M * M; i += blockDim.x)
+        l[i] = g0 * M * M + i < groups * M * M ? lower[int64_t(g0) * M * M + i] : 0.0;
+    __syncthreads();
+    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= per_lane) return;
+    const int64_t xy = per_lane <= 0xffffffffll ? static_cast<unsigned>(k) / static_cast<unsigned>(nzp) : k / nzp;
+    const int64_t zp = k - xy * nzp, p = xy * nz + zp;
+    double x[P * M];
+#pragma unroll
+    for (int i = 0; i < P * M; ++i)
+        x[i] = zp < nz && g0 + i / M < groups ? in[(int64_t(g0) * M + i) * n + p] : 0.0;
+    if (zp < nz) {
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            if (g0 + q >= groups) break;
+            const double* lq = l + q * M * M;
+#pragma unroll
+            for (int i = 0; i < M; ++i) {
+                double v = x[q * M + i];
+#pragma unroll
+                for (int j = 0; j < i; ++j) v -= lq[i * M + j] * x[q * M + j];
+                x[q * M + i] = v / lq[i * M + i];
+                basis[(int64_t(g0 + q) * M + i) * n + p] = x[q * M + i];
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < LANES; ++j) {
+        const int64_t lane = int64_t(g0) * M / 2 + j;
+        if (lane < lane_total) lanes[lane * per_lane + k] = make_double2(x[2 * j], x[2 * j + 1]);
+    }
+}
+
+template <int M>
+int launch_solve_pack(const cdftb_operator* op, const double* lower, const double* block, int64_t batch, double* basis,
+                      void* lanes, cudaStream_t stream) {
+    const int nzp = (op->nz + 1) / 2 * 2;
+    const int64_t per_lane = int64_t(op->nx) * op->ny * nzp;
+    const int groups = static_cast<int>(batch / M);
+    const dim3 grid(static_cast<unsigned>(ceil_div(per_lane, 256)),
+                    static_cast<unsigned>(ceil_div(groups, SolveShape<M>::P)));
+    solve_pack_kernel<M><<<grid, 256, 0, stream>>>(lower, block, groups, int64_t(op->nx) * op->ny * op->nz, per_lane,
+                                                   op->nz, nzp, ceil_div(batch, int64_t(2)), basis,
+                                                   static_cast<double2*>(lanes));
+    return check_launch();
+}
+
+int solve_pack(const cdftb_operator* op, const double* lower, const double* block, int64_t batch, double* basis,
+               void* lanes, cudaStream_t stream) {
+    switch (op->orbitals_per_group) {
+#define CDFTB_SOLVE(M) \
+    case M: return launch_solve_pack<M>(op, lower, block, batch, basis, lanes, stream);
+        CDFTB_SOLVE(1) CDFTB_SOLVE(2) CDFTB_SOLVE(3) CDFTB_SOLVE(4) CDFTB_SOLVE(5) CDFTB_SOLVE(6) CDFTB_SOLVE(7) CDFTB_SOLVE(8)
+#undef CDFTB_SOLVE
+        default: return CDFTB_ERR_ARGUMENT;
+    }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     if (!fn) {
@@ -1791,7 +1867,8 @@ int encode_lanes(void* buf, int nzp, int ny, int nx, int64_t lanes, int ty, int 
         return encode_lane_maps(buf, nzp, ny, nx, lanes, tz, phi, prev);
 }
 
-// The call's copies: the caller's block into lanes at dst, the geometry into padded rows at geo_base.
+// The call's copies: the caller's block (or none) into lanes at dst, the geometry into padded rows at
+// geo_base.
 template <typename L>
 int prepare(const cdftb_operator* op, const void* block, int in_dtype, int64_t batch, int64_t lanes, void* dst,
             void* geo_base, bool without_potential, cudaStream_t stream, const void* scale = nullptr,
@@ -1801,7 +1878,9 @@ int prepare(const cdftb_operator* op, const void* block, int in_dtype, int64_t b
     int64_t blocks = geometry_jobs<L>(op, batch, geo_base, without_potential || !op->potential, inv_fill, &a);
     a.pack_first = blocks;
     const int nzp = padded_z(op->nz);
-    if constexpr (L::WIDE) {
+    if (!block) {
+        // the lanes are written by the caller
+    } else if constexpr (L::WIDE) {
         a.lane_blocks = ceil_div(int64_t(op->nx) * op->ny * nzp, kPrepPerBlock);
         a.block = block;
         a.block_dtype = in_dtype;
@@ -2038,7 +2117,8 @@ int slab_filter(const cdftb_operator* op, const void* block, int in_dtype, void*
 
 template <typename Lane>
 int slab_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* out, int out_dtype, void* work,
-               int64_t batch, int kinetic_only, cudaStream_t stream, const void* scale = nullptr, double inv_fill = 0.0) {
+               int64_t batch, int kinetic_only, cudaStream_t stream, const void* scale = nullptr, double inv_fill = 0.0,
+               const double* lower = nullptr, double* basis = nullptr) {
     const int nx = op->nx, ny = op->ny, nz = op->nz;
     const int nzp = padded_z(nz);
     const int64_t lanes = lane_count<Lane>(op, batch);
@@ -2048,8 +2128,10 @@ int slab_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* ou
     TileChoice choice{t0.ty, t0.tz, 0};
     const TuneKey key = tune_key(op, lanes, Lane::WIDE);
     const bool known = tuned_choice(key, &choice);
-    int st = prepare<Lane>(op, phi, in_dtype, batch, lanes, w, w + lanes * lane_bytes, kinetic_only != 0, stream,
-                           scale, inv_fill);
+    int st = prepare<Lane>(op, lower ? nullptr : phi, in_dtype, batch, lanes, w, w + lanes * lane_bytes,
+                           kinetic_only != 0, stream, scale, inv_fill);
+    // with a factor, of L^{-1} phi (float64 wide lanes in orbital order)
+    if (st == CDFTB_OK && lower) st = solve_pack(op, lower, static_cast<const double*>(phi), batch, basis, w, stream);
     if (st != CDFTB_OK) return st;
     bool autotune;
     {
@@ -2300,4 +2382,28 @@ extern "C" int cdftb_cusp_apply_adjoint_f64(const cdftb_operator* op, const doub
     cdftb::adjoint_finish_kernel<<<static_cast<unsigned>(cdftb::ceil_div(n, 256)), 256, 0, s>>>(
         y, phi, static_cast<const double*>(op->potential), batch, n, phi_bar, potential_bar);
     return cdftb::check_launch();
+}
+
+extern "C" int cdftb_cusp_apply_solved_f64(const cdftb_operator* op, const double* lower, const double* block,
+                                           double* basis, double* out, int64_t batch, void* work, int64_t work_bytes,
+                                           cdftb_stream_t stream) {
+    if (!op || !lower || !block || !basis || !out || op->dtype != CDFTB_F64 || op->orbitals_per_group < 1 || batch < 1 ||
+        batch % op->orbitals_per_group != 0 || op->nx <= 0 || op->ny <= 0 || op->nz <= 0)
+        return CDFTB_ERR_ARGUMENT;
+    const int m = op->orbitals_per_group;
+    const int64_t n = int64_t(op->nx) * op->ny * op->nz, groups = batch / m;
+    const bool fused = m <= 8 && groups <= 65535 && work && cdftb::slab_filter_applies(op) &&
+                       !op->per_system_geometry && cdftb::wide_applies(op, batch) &&
+                       work_bytes >= cdftb_cusp_apply_work_bytes(op, batch) &&
+                       reinterpret_cast<uintptr_t>(work) % 16 == 0 && op->spacing > 0.0 && op->face_weights[0] &&
+                       op->face_weights[1] && op->face_weights[2] && op->inverse_weight && op->potential;
+    if (!fused) {
+        if (groups > 65535) return CDFTB_ERR_ARGUMENT;
+        const int st = cdftb_block_trsm_lower_f64(lower, block, m * n, basis, CDFTB_F64, m * n, m, n,
+                                                  static_cast<int>(groups), stream);
+        if (st != CDFTB_OK) return st;
+        return cdftb_cusp_apply(op, basis, CDFTB_F64, out, CDFTB_F64, batch, 0, work, work_bytes, stream);
+    }
+    return cdftb::slab_apply<cdftb::WideD2>(op, block, CDFTB_F64, out, CDFTB_F64, work, batch, 0, cdftb::as_stream(stream),
+                                            nullptr, 0.0, lower, basis);
 }

@@ -97,6 +97,13 @@ int64_t cdftb_cusp_apply_work_bytes(const cdftb_operator* op, int64_t batch);
 int cdftb_cusp_apply(const cdftb_operator* op, const void* phi, int in_dtype, void* out, int out_dtype,
                      int64_t batch, int kinetic_only, void* work, int64_t work_bytes, cdftb_stream_t stream);
 
+/* basis[g] = L[g]^{-1} block[g] for each group of op->orbitals_per_group orbitals (as
+ * cdftb_block_trsm_lower_f64) and out = A basis, for a float64 operator: the solve writes the apply's lanes
+ * where the order-8 kernel with one geometry takes the call, and is a call of its own elsewhere. Work as
+ * cdftb_cusp_apply. */
+int cdftb_cusp_apply_solved_f64(const cdftb_operator* op, const double* lower, const double* block, double* basis,
+                                double* out, int64_t batch, void* work, int64_t work_bytes, cdftb_stream_t stream);
+
 /* Slab tile of the apply/filter kernels, process-wide: tile_y rows (4, 8 or 16) of 32 z columns per
  * CTA, x chunks no shorter than min_chunk planes, about ctas_per_sm CTAs per SM. Chosen by the
  * host autotuner; no reference counterpart (the reference has no kernels of its own). */
