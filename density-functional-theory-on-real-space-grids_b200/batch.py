@@ -97,7 +97,10 @@ class BatchedHamiltonian:
 
     def apply_solved(self, lower: torch.Tensor, block: torch.Tensor, basis: torch.Tensor) -> torch.Tensor:
         """``basis = L^-1 block`` per system and ``A basis`` (float64), the basis packed as it is formed."""
-        b, k, _ = block.shape
+        b, k, n = block.shape
+        if not (block.dtype == basis.dtype == lower.dtype == self.dtype == torch.float64 and basis.shape == block.shape
+                and lower.shape == (b, k, k) and n == self.grid.n_points and b <= self.batch):
+            raise ValueError("apply_solved takes float64 blocks (B, k, N) and factors (B, k, k) of this operator's systems")
         out = torch.empty_like(block)
         op = self._op(k)
         work = apply_workspace(op, b * k, block.device)

@@ -1419,8 +1419,8 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(const __grid_constan
 // The columns' triangular solve x = L^{-1} b of each group (as trsm_lower_fixed_kernel, bit for bit) that
 // leaves the basis in caller layout and in float64 wide lanes: the block is read once and the basis not
 // read again to be packed. HBM bounds it (3 M values per point and group). A thread takes a point of P
-// groups, so that P M orbitals fill whole lanes. 32 groups of 5 at 65^3: 170 us (HBM at its copy rate: 161), where the solve and
-// the packing took 136 and 100.
+// groups, so that P M orbitals fill whole lanes. 32 groups of 5 at 65^3: 170 us (HBM at its copy rate:
+// 161), where the solve and the packing took 136 and 100.
 template <int M>
 struct SolveShape {
     static constexpr int P = M % 2 ? 2 : 1, LANES = P * M / 2;

@@ -404,6 +404,9 @@ class RitzStep:
         stream = stream_handle(flat.device)
         call("cdftb_ritz_basis_f64", ptr(flat), ptr(q), m, n, ptr(basis), ptr(work), work.numel(), stream)
         applied = hamiltonian.apply(basis).contiguous()
+        if applied.dtype != torch.float64 or applied.shape != basis.shape:
+            raise ValueError(f"the operator's apply gave {tuple(applied.shape)} {applied.dtype} for a float64 block "
+                             f"of {tuple(basis.shape)}")
         vectors = torch.empty_like(flat)
         evals, residuals, summary = torch.empty(2 * m + 5, dtype=torch.float64, device=flat.device).split((m, m, 5))
         call("cdftb_ritz_vectors_f64", ptr(basis), ptr(applied), ptr(q), ptr(previous.contiguous()), n_states, m, n,

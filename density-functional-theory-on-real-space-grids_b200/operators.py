@@ -323,7 +323,7 @@ def lanczos_bounds(hamiltonian: CuspFactoredHamiltonian, start: torch.Tensor, st
     tridiagonal problem is solved on the host, as in the reference.
     """
     if (type(hamiltonian) is CuspFactoredHamiltonian and hamiltonian.dtype == torch.float64 and steps >= 1
-            and start.device.type == "cuda" and start.numel() == hamiltonian.grid.n_points):
+            and start.device == hamiltonian._inv.device and start.numel() == hamiltonian.grid.n_points):
         values = _native_lanczos(hamiltonian, start, steps)
     else:
         values = _lanczos_recurrence(hamiltonian, start, steps)
