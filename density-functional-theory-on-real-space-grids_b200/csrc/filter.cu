@@ -982,7 +982,7 @@ __global__ void __maxnreg__((wide_max_registers<WideShape<TYW, TZ, sizeof(typena
 
     if (warp >= SH::MW) {
         const int pg = (warp - SH::MW) / SH::PWG;
-        if constexpr (!SH::SPLIT) {
+        if constexpr (!SH::SPLIT || GENERAL) {
             const int it = t - (SH::MW + pg * SH::PWG) * 32;
             bool active = false;
             int nb = 0, ns = 0, wb = 0, ws = 0, ob = 0, os = 0, first = 0;
@@ -1050,7 +1050,8 @@ __global__ void __maxnreg__((wide_max_registers<WideShape<TYW, TZ, sizeof(typena
         }
         // Whole warps of one kind: the strides are compile-time offsets of the loads and stores. (In float64
         // the mixed warps above are the faster ones, 24.7 against 28.2 us per step for one He 65^3 system;
-        // in float32, 64 systems, these are, 519 against 549.)
+        // in float32, 64 systems, these are, 519 against 549, but not beside the general form's lookups: 48
+        // systems on their own grids, 13 x 24, 70.2 ms mixed against 85.2 for a solve's 180 steps.)
         auto planes = [&](auto ns, auto ws, auto os, bool active, int nb, int wb, int ob, int first) {
             int s = pg, ph = 0, q = q0 + pg;
             auto next = [&]() {
