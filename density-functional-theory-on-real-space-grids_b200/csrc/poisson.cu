@@ -412,9 +412,10 @@ __global__ void __launch_bounds__(kThreads4) fft_middle_fourstep_kernel(const cp
     }
 }
 
-// Pass 1, four-step: z lines (contiguous, nz real values) -> half spectrum kz < nk. Two real lines a, b
-// share one complex transform of a + i b: with Z its spectrum, A[k] = (Z[k] + conj Z[N-k]) / 2 and
-// B[k] = (Z[k] - conj Z[N-k]) / 2i.
+// Pass 1, four-step: the z lines (contiguous, nz real values) of system blockIdx.y -> half spectrum kz < nk.
+// Two real lines a, b share one complex transform of a + i b: with Z its spectrum,
+// A[k] = (Z[k] + conj Z[N-k]) / 2 and B[k] = (Z[k] - conj Z[N-k]) / 2i. Rounding errors of one line, and its
+// NaN, reach the other one, so the two are always lines of one system (an odd last line has zeros beside it).
 template <int A, int B>
 __global__ void __launch_bounds__(kThreads4) fft_z_forward_fourstep_kernel(const double* __restrict__ rho,
                                                                           int64_t lines, int nz,
@@ -423,7 +424,8 @@ __global__ void __launch_bounds__(kThreads4) fft_z_forward_fourstep_kernel(const
     using F = FourStep<A, B>;
     constexpr int N = F::N, L = kLines4, LP = L + 1;
     __shared__ cplx buf[N * LP];
-    const int64_t l0 = int64_t(blockIdx.x) * (2 * L);
+    const int64_t l0 = blockIdx.y * lines + int64_t(blockIdx.x) * (2 * L);
+    lines *= blockIdx.y + 1;  // the end of the system's lines
 #pragma unroll 4
     for (int idx = threadIdx.x; idx < 2 * L * F::ROWS; idx += kThreads4) {
         const int line = idx / F::ROWS, z = idx % F::ROWS;
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(kThreads4) fft_z_forward_fourstep_kernel(const
     }
 }
 
-// Pass 5, four-step: half spectra -> real z lines (z < nz), two lines per
+// Pass 5, four-step: half spectra -> real z lines (z < nz) of system blockIdx.y, two lines per
 // complex transform of A + i B (both Hermitian-extended; irfft drops the imaginary parts of the k = 0
 // and Nyquist terms, which would leak into the other line here).
 template <int A, int B>
@@ -465,7 +467,8 @@ __global__ void __launch_bounds__(kThreads4) fft_z_inverse_fourstep_kernel(const
     using F = FourStep<A, B>;
     constexpr int N = F::N, L = kLines4, LP = L + 1;
     __shared__ cplx buf[N * LP];
-    const int64_t l0 = int64_t(blockIdx.x) * (2 * L);
+    const int64_t l0 = blockIdx.y * lines + int64_t(blockIdx.x) * (2 * L);
+    lines *= blockIdx.y + 1;  // the end of the system's lines
 #pragma unroll 2
     for (int idx = threadIdx.x; idx < L * nk; idx += kThreads4) {
         const int pair = idx / nk, k = idx - pair * nk;
@@ -1107,12 +1110,12 @@ int run_fourstep(cdftb_poisson_plan* p, const double* density, double* potential
     const int d = pass == 3 ? 0 : (pass == 1 || pass == 5 ? 2 : 1);
     const int A = p->four[d][0], B = p->four[d][1];
     const cplx* twn = p->twn[d];
-    const int64_t lines = static_cast<int64_t>(batch) * nx * ny;
+    const int64_t lines = static_cast<int64_t>(nx) * ny;
     const int64_t inner = static_cast<int64_t>(N1) * nk;
     const int64_t small = static_cast<int64_t>(ny) * nk;
     const dim3 grid = pass == 3 ? dim3(static_cast<unsigned>(ceil_div(inner, kLines4)), static_cast<unsigned>(batch))
                       : d == 1  ? dim3(static_cast<unsigned>(batch * nx), static_cast<unsigned>(ceil_div(nk, kLines4)))
-                                : dim3(static_cast<unsigned>(ceil_div(lines, 2 * kLines4)));
+                                : dim3(static_cast<unsigned>(ceil_div(lines, 2 * kLines4)), static_cast<unsigned>(batch));
 #define CDFTB_X4(A_, B_)                                                                                              \
     if (A == A_ && B == B_) {                                                                                         \
         switch (pass) {                                                                                               \

@@ -280,8 +280,8 @@ int cdftb_poisson_plan_create(int nx, int ny, int nz, double spacing, double pad
 int cdftb_poisson_plan_destroy(void* plan);
 /* The device kernel table K (padded0, padded1, padded2/2+1) of a plan. */
 int cdftb_poisson_kernel_table(void* plan, const double** table);
-/* v = irfftn(rfftn(pad(rho)) K)[:n] for `batch` densities (batch x N each): CoulombCutoffPoisson.solve
- * (poisson.py:66-84). */
+/* v = irfftn(rfftn(pad(rho)) K)[:n] for `batch` densities (batch x N each), each as if it were alone:
+ * CoulombCutoffPoisson.solve (poisson.py:66-84). */
 int cdftb_poisson_solve(void* plan, const double* density, double* potential, int batch, cdftb_stream_t stream);
 
 /* ---- (d) exchange-correlation, spin-restricted (src/cdft/xc/base.py:115-189) ---- */
