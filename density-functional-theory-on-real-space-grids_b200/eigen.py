@@ -384,13 +384,16 @@ class RitzStep:
     For blocks of at most 8 orbitals: two library calls around the apply (``cdftb_ritz_basis_f64``,
     ``cdftb_ritz_vectors_f64``) in place of nine and of a dozen torch launches over m x m numbers, which set the
     pace of a solve on a small grid (33^3, 5 orbitals: 0.6 ms of host work per iteration, 0.35 ms of device work).
-    The work buffer belongs to one solve and its stream.
+    The work buffer belongs to one solve and its stream. The summary's fourth value is that of row ``top``, from
+    which the next filter's interval starts (by default the last row; a wider start block keeps its rows, but the
+    interval starts where that of the wanted and extra states does).
     """
 
     MOST = 8
 
-    def __init__(self, measure: Measure, m: int, device) -> None:
+    def __init__(self, measure: Measure, m: int, device, top: int | None = None) -> None:
         self.m = m
+        self.top = m - 1 if top is None else top
         self.n = measure.grid.n_points
         self.q = measure.quadrature
         nbytes = _lib.library().cdftb_ritz_work_bytes(m, self.n)
@@ -411,6 +414,8 @@ class RitzStep:
         evals, residuals, summary = torch.empty(2 * m + 5, dtype=torch.float64, device=flat.device).split((m, m, 5))
         call("cdftb_ritz_vectors_f64", ptr(basis), ptr(applied), ptr(q), ptr(previous.contiguous()), n_states, m, n,
              ptr(vectors), ptr(evals), ptr(residuals), ptr(summary), ptr(work), work.numel(), stream)
+        if self.top != m - 1:
+            summary[3:4].copy_(evals[self.top:self.top + 1])
         return evals, vectors, residuals, summary
 
 
@@ -523,7 +528,7 @@ class ChebyshevFilteredSubspace:
         top_fraction = float("-inf")
         filt = self.filter_hamiltonian or hamiltonian
         m = vectors.shape[0]
-        ritz = (RitzStep(measure, m, vectors.device)
+        ritz = (RitzStep(measure, m, vectors.device, min(size, m) - 1)
                 if isinstance(measure, Measure) and m <= RitzStep.MOST and 1 <= n_states <= m else None)
         for iteration in range(1, cfg.max_iterations + 1):
             lower = next_lower
