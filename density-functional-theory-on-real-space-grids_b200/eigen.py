@@ -407,7 +407,7 @@ class RitzStep:
         stream = stream_handle(flat.device)
         call("cdftb_ritz_basis_f64", ptr(flat), ptr(q), m, n, ptr(basis), ptr(work), work.numel(), stream)
         applied = hamiltonian.apply(basis).contiguous()
-        if applied.dtype != torch.float64 or applied.shape != basis.shape:
+        if applied.dtype != torch.float64 or applied.numel() != basis.numel():
             raise ValueError(f"the operator's apply gave {tuple(applied.shape)} {applied.dtype} for a float64 block "
                              f"of {tuple(basis.shape)}")
         vectors = torch.empty_like(flat)

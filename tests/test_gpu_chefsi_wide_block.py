@@ -1,4 +1,5 @@
-"""The eigensolver's iteration for start blocks wider than the wanted states and their extra ones."""
+"""The eigensolver's iteration for start blocks wider than the wanted states and their extra ones, and for operators
+that return their result in another shape."""
 
 from __future__ import annotations
 
@@ -15,7 +16,7 @@ def ham(pkg, cuda):
     return geo
 
 
-def _solve(pkg, geo, n_states, block):
+def _solve(pkg, geo, n_states, block, operator=None):
     h = pkg.CuspFactoredHamiltonian(geo.grid, geo.factor, quadrature=geo.quadrature)
     lower = []
 
@@ -24,7 +25,7 @@ def _solve(pkg, geo, n_states, block):
         return pkg.chebyshev_filter(hamiltonian, vectors, degree, low, *bounds)
 
     solver = pkg.ChebyshevFilteredSubspace(geo.grid, pkg.EigenConfig(max_iterations=3), filter_engine=engine)
-    result = solver.solve(h, n_states, initial=block, generator=torch.Generator().manual_seed(5))
+    result = solver.solve(operator(h) if operator else h, n_states, initial=block, generator=torch.Generator().manual_seed(5))
     return lower, result, h
 
 
@@ -41,3 +42,23 @@ def test_filter_bound_is_the_wanted_blocks_top(pkg, cuda, ham, monkeypatch, n_st
     assert len(lower) == 3 and lower == pytest.approx(want_lower, rel=1e-9)
     torch.testing.assert_close(result.eigenvalues, want.eigenvalues, rtol=1e-9, atol=1e-9)
     assert (result.n_iterations, h.apply_count) == (want.n_iterations, want_h.apply_count)
+
+
+class _Reshaping:
+    """An operator whose apply returns ``(1, m, N)``."""
+
+    def __init__(self, inner):
+        self._inner = inner
+
+    def __getattr__(self, name):
+        return getattr(self._inner, name)
+
+    def apply(self, phi):
+        return self._inner.apply(phi)[None]
+
+
+def test_operator_may_return_another_shape(pkg, cuda, ham):
+    block = torch.randn((5, ham.grid.n_points), dtype=torch.float64, generator=torch.Generator().manual_seed(1)).to(cuda)
+    want = _solve(pkg, ham, 1, block)[1]
+    got = _solve(pkg, ham, 1, block, _Reshaping)[1]
+    assert torch.equal(got.eigenvalues, want.eigenvalues)
