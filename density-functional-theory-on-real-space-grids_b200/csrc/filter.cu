@@ -40,6 +40,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "per_device.cuh"
 
 namespace cdftb {
 
@@ -1624,13 +1625,12 @@ int take_test_stop() { return g_test_stop_after.exchange(0, std::memory_order_re
 template <typename Lane, int TZ>
 int launch_slab(const FilterMaps& maps, FilterArgs a, int64_t lanes, cudaStream_t stream, int xchunk = 0) {
     using SH = Shape<TZ, sizeof(typename Lane::S)>;
-    static bool configured = false;
-    if (!configured) {
-        int st = check(cudaFuncSetAttribute(slab_filter_kernel<Lane, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(SH::BYTES)));
-        if (st != CDFTB_OK) return st;
-        configured = true;
-    }
+    static OncePerDevice configured;
+    const int ready = configured.run([] {
+        return check(cudaFuncSetAttribute(slab_filter_kernel<Lane, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(SH::BYTES)));
+    });
+    if (ready != CDFTB_OK) return ready;
     const int tiles_y = static_cast<int>(ceil_div(a.ny, TY));
     a.tiles_z = static_cast<int>(ceil_div(a.nzp, TZ));
     const int64_t tiles = int64_t(tiles_y) * a.tiles_z;
@@ -1774,8 +1774,8 @@ bool g_wide = true;  // guarded by g_tune_mutex (declared below with the tuner)
 template <typename W, int TYW, int TZ, bool GENERAL>
 int launch_wide_as(const FilterMaps& maps, FilterArgs a, int64_t lanes, cudaStream_t stream, int xchunk) {
     using SH = WideShape<TYW, TZ, sizeof(typename W::S), W::ORB>;
-    static bool configured = false;
-    if (!configured) {
+    static OncePerDevice configured;
+    const int ready = configured.run([]() -> int {
         int st = check(cudaFuncSetAttribute(slab_filter_wide_kernel<W, TYW, TZ, GENERAL>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SH::BYTES)));
         if (st != CDFTB_OK) return st;
@@ -1783,9 +1783,9 @@ int launch_wide_as(const FilterMaps& maps, FilterArgs a, int64_t lanes, cudaStre
         cudaFuncAttributes attr{};
         st = check(cudaFuncGetAttributes(&attr, slab_filter_wide_kernel<W, TYW, TZ, GENERAL>));
         if (st != CDFTB_OK) return st;
-        if (attr.maxThreadsPerBlock < SH::T) return CDFTB_ERR_CAPACITY;
-        configured = true;
-    }
+        return attr.maxThreadsPerBlock < SH::T ? CDFTB_ERR_CAPACITY : CDFTB_OK;
+    });
+    if (ready != CDFTB_OK) return ready;
     const int tiles_y = static_cast<int>(ceil_div(a.ny, TYW));
     a.tiles_z = static_cast<int>(ceil_div(a.nzp, TZ));
     const int64_t tiles = int64_t(tiles_y) * a.tiles_z;

@@ -13,6 +13,7 @@
 // order, so the results do not depend on scheduling.
 
 #include "common.cuh"
+#include "per_device.cuh"
 
 namespace cdftb {
 namespace {
@@ -668,13 +669,12 @@ extern "C" int cdftb_quadrature_lift_cells_f64(const void* plan, int64_t plan_by
     if (st != CDFTB_OK) return st;
     int f0 = 0;
     if (nf >= CDFTB_LIFT_CELLS_MANY) {
-        static bool configured = false;
-        if (!configured) {
-            st = check(cudaFuncSetAttribute(lift_cells_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(kManySmem)));
-            if (st != CDFTB_OK) return st;
-            configured = true;
-        }
+        static OncePerDevice configured;
+        st = configured.run([] {
+            return check(cudaFuncSetAttribute(lift_cells_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              static_cast<int>(kManySmem)));
+        });
+        if (st != CDFTB_OK) return st;
         double* rows = static_cast<double*>(scratch);
         double* partial = rows + m * MANY;
         for (; nf - f0 >= CDFTB_LIFT_CELLS_MANY; f0 += MANY) {

@@ -13,6 +13,7 @@
 // src/cdft/operators/hamiltonian.py:303-318 (epilogue), src/cdft/eigen/chefsi.py:81-160 (recurrence).
 
 #include "common.cuh"
+#include "per_device.cuh"
 
 namespace cdftb {
 
@@ -400,13 +401,12 @@ int choose_xchunk(int nx, int64_t ctas_per_plane_set) {
 template <typename T, int P, int TYV>
 int launch_one(const StencilArgs& part, dim3 grid, cudaStream_t stream) {
     using L = StencilLayout<T, P, TYV>;
-    static bool configured = false;  // one attribute call per instantiation and process
-    if (!configured) {
-        int st = check(cudaFuncSetAttribute(stencil_kernel<T, P, TYV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(L::BYTES)));
-        if (st != CDFTB_OK) return st;
-        configured = true;
-    }
+    static OncePerDevice configured;
+    const int ready = configured.run([] {
+        return check(cudaFuncSetAttribute(stencil_kernel<T, P, TYV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(L::BYTES)));
+    });
+    if (ready != CDFTB_OK) return ready;
     stencil_kernel<T, P, TYV><<<grid, dim3(TZ, TYV), L::BYTES, stream>>>(part);
     return check_launch();
 }
