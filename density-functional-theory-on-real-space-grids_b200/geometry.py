@@ -379,7 +379,8 @@ class CuspQuadrature:
 
     # --- interpolation and its transpose (quadrature.py:613-650) ---
     #: The entry lists of L^T (cdftb_lift_plan_build and its values and segments), which the C entry points
-    #: over them take and the lift here does not: built when first read.
+    #: over them take and the lift here does not: built when first read, on the current stream, which is then
+    #: waited for (another stream may use them at once). So the first read must not lie inside a stream capture.
     _CSR = ("row_ptr", "col", "lift_values", "seg_ptr", "seg_row", "seg_capacity")
 
     def __getattr__(self, name):
@@ -403,6 +404,7 @@ class CuspQuadrature:
         scratch = torch.empty(lib.cdftb_lift_segments_scratch_bytes(n), dtype=torch.uint8, device=dev)
         call("cdftb_lift_plan_segments", ptr(row_ptr), *shape, ptr(seg_ptr), ptr(seg_row), capacity, ptr(scratch),
              scratch.numel(), stream)
+        torch.cuda.current_stream(dev).synchronize()
         self.row_ptr, self.col, self.lift_values = row_ptr, col, values
         self.seg_ptr, self.seg_row, self.seg_capacity = seg_ptr, seg_row, capacity
         return self.__dict__[name]
