@@ -54,7 +54,23 @@ struct CellPlan {
     double* w_sorted;    // 24 weights per sorted node
     int *few_ptr, *few_block, *many_ptr, *many_block;  // a block's first item; an item's block
     int64_t bytes;
+    // The plan's first words: how many of its nodes failed the build's check (none in a plan that may be used),
+    // and the key of the sizes and box it was built for. The kernels compare the key with their call's before they
+    // follow anything in the plan, so that a plan that failed, or another call's, is never followed out of range.
+    unsigned long long *bad, *built;
+    unsigned long long key;
 };
+
+__device__ __forceinline__ bool usable(const CellPlan& p) { return *p.built == p.key; }
+
+// A key of the sizes and the box (FNV-1a over them, never zero).
+unsigned long long plan_key(const CellPlan& p) {
+    const int64_t words[] = {p.m, p.nx, p.ny, p.nz, p.lo[0], p.lo[1], p.lo[2], p.hi[0], p.hi[1], p.hi[2]};
+    unsigned long long h = 14695981039346656037ull;
+    for (const int64_t w : words)
+        for (int byte = 0; byte < 8; ++byte) h = (h ^ ((static_cast<unsigned long long>(w) >> (8 * byte)) & 255)) * 1099511628211ull;
+    return h | 1;
+}
 
 template <typename S>
 Blocks blocks_of(const CellPlan& p) {
@@ -98,6 +114,9 @@ bool plan_layout(int64_t m, int nx, int ny, int nz, const int* cell_box, void* b
         at += (bytes + 255) / 256 * 256;
         return r;
     };
+    p.bad = reinterpret_cast<unsigned long long*>(take(16));
+    p.built = p.bad + 1;
+    p.key = plan_key(p);
     p.w_sorted = reinterpret_cast<double*>(take(m * kRow * 8));
     p.cell_ptr = reinterpret_cast<int*>(take((cells + 1) * 4));
     p.order = reinterpret_cast<int*>(take(m * 4));
@@ -125,17 +144,27 @@ __global__ void cell_starts_kernel(const int64_t* __restrict__ keys, int64_t m, 
     cell_ptr[c] = static_cast<int>(lo);
 }
 
+// The weights, node and z cell of every sorted node, which is checked on the way: the runs and items take for
+// granted that the keys ascend, that each is its node's cell, and that no cell lies outside the box.
 __global__ void sort_nodes_kernel(const int* __restrict__ base, const double* __restrict__ w1d,
-                                  const int* __restrict__ order, const CellPlan p) {
+                                  const int* __restrict__ order, const int64_t* __restrict__ keys, const CellPlan p) {
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= p.m * kRow) return;
     const int64_t i = k / kRow;
     const int c = static_cast<int>(k - i * kRow);
     const int node = order[i];
+    if (node < 0 || node >= p.m) {
+        if (c == 0) atomicAdd(p.bad, 1ull);
+        return;
+    }
     p.w_sorted[k] = w1d[int64_t(node) * kRow + c];
     if (c == 0) {
+        const int x = base[int64_t(node) * 3], y = base[int64_t(node) * 3 + 1], z = base[int64_t(node) * 3 + 2];
+        const bool inside = x >= p.lo[0] && x <= p.hi[0] && y >= p.lo[1] && y <= p.hi[1] && z >= p.lo[2] && z <= p.hi[2];
+        if (!inside || keys[i] != (int64_t(x) * p.ny + y) * p.nz + z || (i > 0 && keys[i - 1] > keys[i]))
+            atomicAdd(p.bad, 1ull);
         p.order[i] = node;
-        p.z_sorted[i] = base[int64_t(node) * 3 + 2];
+        p.z_sorted[i] = z;
     }
 }
 
@@ -160,7 +189,7 @@ __device__ __forceinline__ void run_range(const CellPlan& p, int x0, int y0, int
     count = p.cell_ptr[row + zb + 1] - first;
 }
 
-// Items per block (into ptr[block]), one warp per block.
+// Items per block (into ptr[block]; none in a plan that failed the check), one warp per block.
 template <typename S>
 __global__ void item_counts_kernel(const CellPlan p, const Blocks b, int* __restrict__ ptr) {
     const int64_t block = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
@@ -168,7 +197,7 @@ __global__ void item_counts_kernel(const CellPlan p, const Blocks b, int* __rest
     if (block >= b.count) return;
     int x0, y0, z0, nodes = 0;
     block_origin<S>(b, static_cast<int>(block), x0, y0, z0);
-    for (int r = lane; r < S::RUNS; r += 32) {
+    for (int r = *p.bad ? S::RUNS : lane; r < S::RUNS; r += 32) {
         int first, count;
         run_range<S>(p, x0, y0, z0, r, first, count);
         nodes += count;
@@ -178,8 +207,9 @@ __global__ void item_counts_kernel(const CellPlan p, const Blocks b, int* __rest
     if (lane == 0) ptr[block] = (nodes + S::NODES - 1) / S::NODES;
 }
 
-// ptr[block] := the items of the blocks before it, ptr[count] := all items; item_block: by one CTA.
-__global__ void __launch_bounds__(1024) item_scan_kernel(int* __restrict__ ptr, int64_t count,
+// ptr[block] := the items of the blocks before it, ptr[count] := all items; item_block: by one CTA, which
+// then marks the plan as built if its nodes passed the check.
+__global__ void __launch_bounds__(1024) item_scan_kernel(const CellPlan p, int* __restrict__ ptr, int64_t count,
                                                          int* __restrict__ item_block) {
     __shared__ int warp_sum[32];
     __shared__ int carry;
@@ -208,7 +238,10 @@ __global__ void __launch_bounds__(1024) item_scan_kernel(int* __restrict__ ptr, 
         if (threadIdx.x == blockDim.x - 1) carry = first + own;
         __syncthreads();
     }
-    if (threadIdx.x == 0) ptr[count] = carry;
+    if (threadIdx.x == 0) {
+        ptr[count] = carry;
+        *p.built = *p.bad ? 0 : p.key;
+    }
 }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -349,8 +382,8 @@ __global__ void __launch_bounds__(FewShape::WARPS * 32)
     __shared__ double red[S::WARPS][NF][S::POINTS];
     __shared__ Runs<S> runs;
     const int item = blockIdx.x;
-    if (item >= p.few_ptr[p.few.count]) return;
-    const int block = p.few_block[item];
+    const int items = p.few_ptr[p.few.count], block = p.few_block[item];
+    if (!usable(p) || item >= items) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int x0, y0, z0;
     block_origin<S>(p.few, block, x0, y0, z0);
@@ -416,7 +449,8 @@ __global__ void __launch_bounds__(FewShape::WARPS * 32)
     }
 }
 
-// out[f] at the block's points: the block's items in order (none: zero). One CTA per block and field.
+// out[f] at the block's points: the block's items in order (none: zero; NaN for a plan that is not this
+// call's). One CTA per block and field.
 template <int NF>
 __global__ void __launch_bounds__(FewShape::POINTS) lift_cells_few_sum_kernel(const CellPlan p,
                                                                               const double* __restrict__ partial,
@@ -428,10 +462,12 @@ __global__ void __launch_bounds__(FewShape::POINTS) lift_cells_few_sum_kernel(co
     block_origin<S>(p.few, block, x0, y0, z0);
     const int px = x0 + ((k & 31) >> 3), py = y0 + (k >> 5), pz = z0 + (k & 7);
     const double* src = partial + f * S::POINTS + k;
-    const int last = p.few_ptr[block + 1];
-    double sum = 0.0;
+    const int first = p.few_ptr[block], end = p.few_ptr[block + 1];
+    const bool ok = usable(p);
+    const int last = ok ? end : first;
+    double sum = ok ? 0.0 : nan("");
 #pragma unroll 4
-    for (int item = p.few_ptr[block]; item < last; ++item) sum += src[int64_t(item) * (NF * S::POINTS)];
+    for (int item = first; item < last; ++item) sum += src[int64_t(item) * (NF * S::POINTS)];
     if (px < p.nx && py < p.ny && pz < p.nz) out[f * out_stride + (int64_t(px) * p.ny + py) * p.nz + pz] = sum;
 }
 
@@ -468,8 +504,8 @@ __global__ void __launch_bounds__(ManyShape::WARPS * 32, 2)
     __shared__ Runs<S> runs;
     double* red = reinterpret_cast<double*>(smem_raw);  // the sums reuse the stages' memory
     const int item = blockIdx.x;
-    if (item >= p.many_ptr[p.many.count]) return;
-    const int block = p.many_block[item];
+    const int items = p.many_ptr[p.many.count], block = p.many_block[item];
+    if (!usable(p) || item >= items) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* stage = red + warp * (2 * kManyStage + kManyWxy);
     double* wxy = stage + 2 * kManyStage;
@@ -554,8 +590,8 @@ __global__ void __launch_bounds__(ManyShape::WARPS * 32, 2)
     }
 }
 
-// out[f] at the block's 32 points: the block's items in order. One CTA per block; the sums pass through
-// a shared tile so that the field-major stores run along z.
+// out[f] at the block's 32 points: the block's items in order (NaN for a plan that is not this call's).
+// One CTA per block; the sums pass through a shared tile so that the field-major stores run along z.
 __global__ void __launch_bounds__(256) lift_cells_many_sum_kernel(const CellPlan p, const double* __restrict__ partial,
                                                                   int nf, double* __restrict__ out,
                                                                   int64_t out_stride) {
@@ -563,9 +599,11 @@ __global__ void __launch_bounds__(256) lift_cells_many_sum_kernel(const CellPlan
     static_assert(S::POINTS == 32, "a tile of 32 points by 32 fields");
     __shared__ double tile[S::POINTS][MANY + 1];
     const int block = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int first = p.many_ptr[block], last = p.many_ptr[block + 1];
+    const int first = p.many_ptr[block], end = p.many_ptr[block + 1];
+    const bool ok = usable(p);
+    const int last = ok ? end : first;
     for (int pt = warp; pt < S::POINTS; pt += 8) {
-        double sum = 0.0;
+        double sum = ok ? 0.0 : nan("");
 #pragma unroll 4
         for (int item = first; item < last; ++item) sum += partial[(int64_t(item) * S::POINTS + pt) * MANY + lane];
         tile[pt][lane] = sum;
@@ -579,13 +617,14 @@ __global__ void __launch_bounds__(256) lift_cells_many_sum_kernel(const CellPlan
 }
 
 // x[f][order[i]] (f < nf) -> rows[i][f], zero for f >= nf: the field values of a sorted node as one row.
-__global__ void __launch_bounds__(256) sorted_rows_kernel(const double* __restrict__ x, int nf, int64_t stride,
-                                                          const int* __restrict__ order, int64_t m,
-                                                          double* __restrict__ rows) {
+__global__ void __launch_bounds__(256) sorted_rows_kernel(const CellPlan p, const double* __restrict__ x, int nf,
+                                                          int64_t stride, double* __restrict__ rows) {
     __shared__ double tile[MANY][MANY + 1];
+    const int64_t m = p.m;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t i0 = int64_t(blockIdx.x) * MANY;
-    const int64_t node = i0 + tx < m ? order[i0 + tx] : 0;
+    const int64_t node = i0 + tx < m ? p.order[i0 + tx] : 0;
+    if (!usable(p)) return;
     for (int f = ty; f < MANY; f += 8) tile[f][tx] = (f < nf && i0 + tx < m) ? x[f * stride + node] : 0.0;
     __syncthreads();
     for (int r = ty; r < MANY; r += 8)
@@ -597,7 +636,7 @@ int build_items(const CellPlan& p, const Blocks& b, int* ptr, int* item_block, c
     item_counts_kernel<S><<<static_cast<unsigned>(ceil_div(b.count * 32, 256)), 256, 0, s>>>(p, b, ptr);
     int st = check_launch();
     if (st != CDFTB_OK) return st;
-    item_scan_kernel<<<1, 1024, 0, s>>>(ptr, b.count, item_block);
+    item_scan_kernel<<<1, 1024, 0, s>>>(p, ptr, b.count, item_block);
     return check_launch();
 }
 
@@ -634,10 +673,11 @@ extern "C" int cdftb_cell_plan_build(const int* base, const double* w1d, const i
         return CDFTB_ERR_ARGUMENT;
     const int64_t cells = int64_t(nx) * ny * nz;
     cudaStream_t s = as_stream(stream);
-    cell_starts_kernel<<<static_cast<unsigned>(ceil_div(cells + 1, 256)), 256, 0, s>>>(keys, m, cells, p.cell_ptr);
-    int st = check_launch();
+    int st = check(cudaMemsetAsync(p.bad, 0, 16, s));
     if (st != CDFTB_OK) return st;
-    sort_nodes_kernel<<<static_cast<unsigned>(ceil_div(m * kRow, 256)), 256, 0, s>>>(base, w1d, order, p);
+    cell_starts_kernel<<<static_cast<unsigned>(ceil_div(cells + 1, 256)), 256, 0, s>>>(keys, m, cells, p.cell_ptr);
+    if ((st = check_launch()) != CDFTB_OK) return st;
+    sort_nodes_kernel<<<static_cast<unsigned>(ceil_div(m * kRow, 256)), 256, 0, s>>>(base, w1d, order, keys, p);
     if ((st = check_launch()) != CDFTB_OK) return st;
     if ((st = build_items<FewShape>(p, p.few, p.few_ptr, p.few_block, s)) != CDFTB_OK) return st;
     return build_items<ManyShape>(p, p.many, p.many_ptr, p.many_block, s);
@@ -680,7 +720,7 @@ extern "C" int cdftb_quadrature_lift_cells_f64(const void* plan, int64_t plan_by
         for (; nf - f0 >= CDFTB_LIFT_CELLS_MANY; f0 += MANY) {
             const int count = nf - f0 < MANY ? nf - f0 : MANY;
             sorted_rows_kernel<<<static_cast<unsigned>(ceil_div(m, MANY)), 256, 0, s>>>(
-                node_values + f0 * x_stride, count, x_stride, p.order, m, rows);
+                p, node_values + f0 * x_stride, count, x_stride, rows);
             if ((st = check_launch()) != CDFTB_OK) return st;
             lift_cells_many_kernel<<<static_cast<unsigned>(p.many.items), ManyShape::WARPS * 32, kManySmem, s>>>(
                 p, rows, partial);

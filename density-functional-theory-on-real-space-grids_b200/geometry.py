@@ -325,7 +325,9 @@ class CuspQuadrature:
         starts = torch.cumsum(counts, 0) - counts
         items = (counts + self.GROUP_BATCH - 1) // self.GROUP_BATCH
         first = torch.repeat_interleave(starts, items)
-        k = torch.arange(int(items.sum()), device=dev) - torch.repeat_interleave(torch.cumsum(items, 0) - items, items)
+        if misplaced := int(self._cell_plan[:8].view(torch.int64)):
+            raise ValueError(f"{misplaced} quadrature nodes lie outside the spheres' box of cells")
+        k = torch.arange(first.numel(), device=dev) - torch.repeat_interleave(torch.cumsum(items, 0) - items, items)
         item_start = first + k * self.GROUP_BATCH
         self.group_ptr = torch.cat([item_start, counts.sum().reshape(1)]).to(torch.int32).contiguous()
         self.n_groups = int(item_start.numel())

@@ -409,7 +409,10 @@ int cdftb_quadrature_lift_many_f64(const long long* row_ptr, const int* col, con
  * cell, int64, ascending; order: the node of every sorted position). cell_box: 6 host ints, per axis
  * the lowest and then the highest cell index that may hold a node. The plan (cdftb_cell_plan_bytes of
  * device memory, 16-byte aligned) keeps each cell's first node, the sorted nodes' weights and the work
- * items of the two kernels. Results equal cdftb_quadrature_lift_f64's up to the order of the sums
+ * items of the two kernels. The build checks the nodes on the device: the plan's first 64-bit word then
+ * holds how many of them have a key below the one before, a key that is not their cell's, a cell outside
+ * the box or an order entry that is no node. A lift with a plan where that is not 0, or with other sizes or
+ * another box than the plan was built for, gives NaN at the points its box reaches. Results equal cdftb_quadrature_lift_f64's up to the order of the sums
  * (~1e-16 relative). From CDFTB_LIFT_CELLS_MANY fields on, a pass takes 32 fields. */
 #define CDFTB_LIFT_CELLS_MANY 8
 int64_t cdftb_cell_plan_bytes(int64_t m, int nx, int ny, int nz, const int* cell_box);
