@@ -790,10 +790,8 @@ int configure_lines() {
 }
 
 int configure_poisson_kernels() {
-    int st = configure_lines<16>();
-    if (st == CDFTB_OK) st = configure_lines<8>();
-    if (st == CDFTB_OK) st = configure_lines<4>();
-    return st;
+    const int st = configure_lines<8>();
+    return st == CDFTB_OK ? configure_lines<4>() : st;
 }
 
 // cos(2 pi j / n) in long double, the angle reduced to a small one exactly in integers.
@@ -1148,10 +1146,8 @@ extern "C" int cdftb_poisson_solve(void* plan, const double* density, double* po
             continue;
         }
         const int n = p->len[axis_of_pass[pass]];
-        const int lines = lines_for(n);
-        const int st = lines == 16  ? run_passes<16>(p, density, potential, batch, s, pass)
-                       : lines == 8 ? run_passes<8>(p, density, potential, batch, s, pass)
-                                    : run_passes<4>(p, density, potential, batch, s, pass);
+        const int st = lines_for(n) == 8 ? run_passes<8>(p, density, potential, batch, s, pass)
+                                         : run_passes<4>(p, density, potential, batch, s, pass);
         if (st != CDFTB_OK) return st;
     }
     return CDFTB_OK;

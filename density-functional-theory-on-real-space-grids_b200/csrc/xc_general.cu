@@ -2,8 +2,9 @@
 // its first derivatives. The reference writes each functional once as an energy density of the
 // per-spin ingredients (n_up, n_dn, sigma_uu, sigma_ud, sigma_dd) and differentiates it with
 // autograd (src/cdft/xc/base.py:115-189); here the same energy densities are evaluated on
-// forward-mode dual numbers that carry all five partial derivatives at once, so v_xc and v_sigma
-// are exact derivatives of the energy density (to rounding), with no hand-derived formula.
+// forward-mode dual numbers, so v_xc and v_sigma are exact derivatives of the energy density (to
+// rounding). An LDA carries its two density partials through; a GGA is assembled from parts of two or
+// three variables, each with the partials of those, which the chain rule joins (Gga below).
 //
 // Conventions kept from base.py:45-80, 171-189:
 //   - n_spin = 1: n_up = n_dn = n/2 and sigma_uu = sigma_ud = sigma_dd = sigma/4; n_spin = 2: the
@@ -195,11 +196,6 @@ __device__ __forceinline__ Dual<N> fourth(const Dual<N>& x) {
     return chain(x2 * x2, 4.0 * (x2 * x.v), x);
 }
 template <int N>
-__device__ __forceinline__ Dual<N> pow13(const Dual<N>& x) {
-    const double c = cbrt(x.v);
-    return chain(c, c / (3.0 * x.v), x);
-}
-template <int N>
 __device__ __forceinline__ Dual<N> pow23(const Dual<N>& x) {
     const double c = cbrt(x.v);
     return chain(c * c, (2.0 / 3.0) / c, x);
@@ -248,8 +244,8 @@ __device__ __forceinline__ Dual<N> f_zeta(const Dual<N>& z) {
 }
 constexpr double kFpp0 = 4.0 / (9.0 * (kCbrt2X - 1.0));
 
-// para + alpha f (1 - z^4) / f''(0) + (ferro - para) f z^4. Without POL the channels are equal: f, f' and
-// z are zero, and the para part is all of it.
+// para + alpha f (1 - z^4) / f''(0) + (ferro - para) f z^4. (With equal channels f, f' and z are zero and the
+// para part is all of it: the callers' POL = false.)
 template <int N>
 __device__ __forceinline__ Dual<N> interpolate_spin(const Dual<N>& para, const Dual<N>& ferro,
                                                     const Dual<N>& alpha_c, const Dual<N>& zeta, double fpp0) {
