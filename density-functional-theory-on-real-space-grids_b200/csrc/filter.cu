@@ -631,8 +631,8 @@ __global__ void __launch_bounds__(Shape<TZ, sizeof(typename Lane::S)>::T, 1)
 //               of them, the newest output opens with its first face, and the oldest one is complete
 //               after its last face, when its plane's y+z part joins it. The pass groups thus have
 //               7 planes of lead on the march, and the result ring is 8 (or 6) slots deep.
-// Lanes run over the orbitals in order (lane l: orbitals ORB l .. ORB l + ORB - 1); lanes aligned to
-// orbital groups (per-system geometry) keep slab_filter_kernel.
+// Lanes run over the orbitals in order (lane l: orbitals ORB l .. ORB l + ORB - 1) or, with a geometry per
+// system, are aligned to the orbital groups (GENERAL; lane_orbital).
 
 struct WideF4 {  // four float32 orbitals
     using E = float4;
@@ -1805,13 +1805,14 @@ int launch_wide_as(const FilterMaps& maps, FilterArgs a, int64_t lanes, cudaStre
 }
 
 // Lanes aligned to orbital groups (per-system geometry) take the general instantiation, and so do
-// the float64 lanes in 8-row tiles: there the general kernels keep every value in registers, where
-// the in-order ones spill 4 bytes (16 He 65^3 systems, 8 x 36: 257.7 against 262.1 us per step).
-// Elsewhere the in-order kernels are the faster ones (float32, 128 systems, 13 x 24: 1102 against
-// 1124 us; float64, one system, 13 x 24: 33.3 against 34.1 us).
+// the float64 lanes in 8 x 36 tiles (16 He 65^3 systems: 264 us per step against 266 in order; one system:
+// 32.1 both ways). Elsewhere the in-order kernels are the faster ones; us per step, general against in order:
+// float64 8 x 32 282 : 277 (261 orbitals at 43 x 39 x 52) and 58.3 : 57.3 (81 x 81 x 91, 5 orbitals), 13 x 24
+// 312 : 290 (16 He 65^3 systems), where the general one spills; float32 8 x 32 55.7 : 53.5 (40 orbitals at
+// 66 x 55 x 53), 8 x 36 312 : 301 (32 He 65^3 systems), 13 x 24 1115 : 1043 (128 of them).
 template <typename W, int TYW, int TZ>
 int launch_wide(const FilterMaps& maps, const FilterArgs& a, int64_t lanes, cudaStream_t stream, int xchunk = 0) {
-    if constexpr (W::ORB == 2 && TYW == 8) {
+    if constexpr (W::ORB == 2 && TYW == 8 && TZ == 36) {
         return launch_wide_as<W, TYW, TZ, true>(maps, a, lanes, stream, xchunk);
     } else {
         return a.lanes_per_group > 0 ? launch_wide_as<W, TYW, TZ, true>(maps, a, lanes, stream, xchunk)
@@ -2193,7 +2194,7 @@ __global__ void __launch_bounds__(256) adjoint_finish_kernel(const double* __res
     if (potential_bar) potential_bar[p] = sum;
 }
 
-// Wide lanes serve every filter and apply with one shared geometry (lanes need not follow orbital
+// Wide lanes serve every filter and apply (with a geometry per system, aligned to the orbital
 // groups). Measured on He 65^3 they were faster at every batch tried, from one system of 5 orbitals
 // (2 or 3 wide lanes) to 32 systems.
 bool wide_applies(const cdftb_operator* op, int64_t batch) {

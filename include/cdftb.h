@@ -126,8 +126,8 @@ int cdftb_chebyshev_filter(const cdftb_operator* op, const void* block, int in_d
 
 /* No reference counterpart (the reference has no kernels of its own to tune): the tile autotuner of
  * the order-8 slab kernels. With it enabled, the first cdftb_chebyshev_filter or cdftb_cusp_apply
- * call for a (device, grid, precision, lane count) key times each candidate tiling -- z tiles of 32
- * or 36 columns, 1 to 7 x chunks and the heuristic's chunk -- on that call's own buffers, keeps the
+ * call for a (device, grid, precision, lane count) key times each candidate tiling -- tiles of 8 rows by 32
+ * or 36 z columns, for wide lanes also 13 by 24, 1 to 7 x chunks and the heuristic's chunk -- on that call's own buffers, keeps the
  * fastest, and every later filter or apply launch for the key uses it. That first call synchronises
  * its stream (make it before any stream capture); results are bit-identical whatever the tiling. Disabled (the
  * default in the C library), heuristics choose the tiling. cdftb_filter_tuned_tile reports the
@@ -143,11 +143,11 @@ int cdftb_filter_tuned_tile(int nx, int ny, int nz, int dtype, int64_t lanes, in
 int cdftb_filter_tuned_tile_rows(int nx, int ny, int nz, int dtype, int64_t lanes, int* tile_y);
 
 /* No reference counterpart: wide lanes for cdftb_chebyshev_filter and cdftb_cusp_apply. Enabled
- * (the default), every order-8 call with one shared geometry (no per-system geometry) runs a
- * kernel that holds 16 bytes per lane point -- four float32 or two float64 orbitals -- instead of
- * 8: the same operator and recurrence, its sums in another order (results differ from the
- * 8-byte-lane kernel by rounding). Calls with per-system geometry, or all calls when disabled, use
- * the 8-byte lanes. The work-size queries cover both layouts. */
+ * (the default), every order-8 call runs a kernel that holds 16 bytes per lane point -- four float32
+ * or two float64 orbitals, with a geometry per system those of one orbital group -- instead of 8: the
+ * same operator and recurrence, its sums in another order (results differ from the 8-byte-lane
+ * kernel by rounding). Disabled, all calls use the 8-byte lanes. The work-size queries cover both
+ * layouts. */
 int cdftb_filter_wide(int enable);
 
 /* No reference counterpart: the error flags the library's kernels set on the device (bit 0: a
