@@ -126,15 +126,14 @@ int cdftb_chebyshev_filter(const cdftb_operator* op, const void* block, int in_d
 
 /* No reference counterpart (the reference has no kernels of its own to tune): the tile autotuner of
  * the order-8 slab kernels. With it enabled, the first cdftb_chebyshev_filter or cdftb_cusp_apply
- * call for a (device, grid, precision, lane count) key times each candidate tiling -- tiles of 8 rows by 32
- * or 36 z columns, for wide lanes also 13 by 24, 1 to 7 x chunks and the heuristic's chunk -- on that call's own buffers, keeps the
- * fastest, and every later filter or apply launch for the key uses it. That first call synchronises
- * its stream (make it before any stream capture); results are bit-identical whatever the tiling. Disabled (the
- * default in the C library), heuristics choose the tiling. cdftb_filter_tuned_tile reports the
- * table's entry for a key (tile_z 32, 36 or 24, x_chunk in planes; both 0 when the key is not tuned)
- * and cdftb_filter_tuned_tile_rows its tile rows (8, or 13 for the wide kernel's 13 x 24 tile; 0 when
- * not tuned);
- * dtype is CDFTB_F32 or CDFTB_F64 and lanes is the launch's lane count (cdftb_operator orbitals in
+ * call for a (device, grid, precision, lane count) key times each candidate tiling -- tiles of 8 rows
+ * by 32 or 36 z columns, for wide lanes also 13 by 24, 1 to 7 x chunks and the heuristic's chunk --
+ * on that call's own buffers, keeps the fastest, and every later filter or apply launch for the key
+ * uses it. That first call synchronises its stream (make it before any stream capture); results are
+ * bit-identical whatever the tiling. Disabled (the default in the C library), heuristics choose the
+ * tiling. cdftb_filter_tuned_tile reports the table's entry for a key (tile_z 32, 36 or 24, x_chunk in
+ * planes; both 0 when the key is not tuned) and cdftb_filter_tuned_tile_rows its tile rows (8, or 13
+ * for the wide kernel's 13 x 24 tile; 0 when not tuned); dtype is CDFTB_F32 or CDFTB_F64 and lanes is the launch's lane count (cdftb_operator orbitals in
  * pairs for float32, one each for float64); for the wide-lane kernels (cdftb_filter_wide) dtype is
  * CDFTB_F32 + CDFTB_WIDE_LANES or CDFTB_F64 + CDFTB_WIDE_LANES and lanes counts four float32 or two
  * float64 orbitals each. */
@@ -412,8 +411,9 @@ int cdftb_quadrature_lift_many_f64(const long long* row_ptr, const int* col, con
  * items of the two kernels. The build checks the nodes on the device: the plan's first 64-bit word then
  * holds how many of them have a key below the one before, a key that is not their cell's, a cell outside
  * the box or an order entry that is no node. A lift with a plan where that is not 0, or with other sizes or
- * another box than the plan was built for, gives NaN at the points its box reaches. Results equal cdftb_quadrature_lift_f64's up to the order of the sums
- * (~1e-16 relative). From CDFTB_LIFT_CELLS_MANY fields on, a pass takes 32 fields. */
+ * another box than the plan was built for, gives NaN at the points its box reaches. Results equal
+ * cdftb_quadrature_lift_f64's up to the order of the sums (~1e-16 relative). From CDFTB_LIFT_CELLS_MANY
+ * fields on, a pass takes 32 fields. */
 #define CDFTB_LIFT_CELLS_MANY 8
 int64_t cdftb_cell_plan_bytes(int64_t m, int nx, int ny, int nz, const int* cell_box);
 int cdftb_cell_plan_build(const int* base, const double* w1d, const int* order, const int64_t* keys, int64_t m,
